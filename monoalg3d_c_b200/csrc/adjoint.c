@@ -26,10 +26,10 @@
 #include "mb_internal.h"
 #include "mb_tissue.h"
 
-int mbk_adj_tt2006(const mb_ode_dev *o, const mb_ctrl *ctrl_n, const double *v_n, const double *sv_n,
+int mbk_adj_tt2006(const mb_ode_dev *o, const double *v_n, const double *sv_n,
                    const double *w, double alpha, const double *mu_in, double *mu_out, double *lam_out,
                    double *gth, cudaStream_t s);
-int mbk_adj_tt2006_mixed(const mb_ode_dev *o, const mb_ctrl *ctrl_n, const double *v_n, const double *sv64_n,
+int mbk_adj_tt2006_mixed(const mb_ode_dev *o, const double *v_n, const double *sv64_n,
                          const float *sv32_n, const double *w, double alpha, const double *mu_in, double *mu_out,
                          double *lam_out, double *gth, cudaStream_t s);
 int mbk_adj_face_grad(const mb_stencil_dev *st, const double *sigma, const double *w, const double *v,
@@ -212,10 +212,9 @@ int mb_adjoint_backward(mb_adjoint *a, const double *dtraces, double *grad_sigma
                     AKK(mbk_adj_scatter(a->d_lam, a->d_sensors, a->ns, a->d_g + (size_t)sample * a->ns, s));
             }
             double *v1, *v0, *sv0;
-            mb_ctrl *c0;
             void *snap0 = a->d_seg + a->snap * (size_t)k;
             mb_tissue_snapshot_parts(m, a->d_seg + a->snap * (size_t)(k + 1), &v1, NULL, NULL);
-            mb_tissue_snapshot_parts(m, snap0, &v0, &sv0, &c0);
+            mb_tissue_snapshot_parts(m, snap0, &v0, &sv0, NULL);
             /* A w = lambda_{step+1} (warm start from the previous w) */
             AKK(mbk_adj_tol(a->d_lam, n, 1e-24, a->d_actrl, s));
             AKK(mbk_fcg_launch(&q, s));
@@ -224,10 +223,10 @@ int mb_adjoint_backward(mb_adjoint *a, const double *dtraces, double *grad_sigma
             /* through the Rush-Larsen step at (v_step, s_step) */
             ACK(cudaMemsetAsync(a->d_lam2, 0, nb, s));
             if (m->desc.precision == MB_PREC_MIXED)
-                AKK(mbk_adj_tt2006_mixed(&o, c0, v0, sv0, mb_tissue_snapshot_sv32(m, snap0), a->d_w, a->alpha,
+                AKK(mbk_adj_tt2006_mixed(&o, v0, sv0, mb_tissue_snapshot_sv32(m, snap0), a->d_w, a->alpha,
                                          a->d_mu, a->d_mu2, a->d_lam2, a->d_gth, s));
             else
-                AKK(mbk_adj_tt2006(&o, c0, v0, sv0, a->d_w, a->alpha, a->d_mu, a->d_mu2, a->d_lam2, a->d_gth, s));
+                AKK(mbk_adj_tt2006(&o, v0, sv0, a->d_w, a->alpha, a->d_mu, a->d_mu2, a->d_lam2, a->d_gth, s));
             double *t = a->d_lam; a->d_lam = a->d_lam2; a->d_lam2 = t;
             t = a->d_mu; a->d_mu = a->d_mu2; a->d_mu2 = t;
             q.b = a->d_lam;

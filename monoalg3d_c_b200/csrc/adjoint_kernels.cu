@@ -9,10 +9,10 @@
 //     A w = lambda_{n+1}                          (A is symmetric: the same PCG)
 //     dL/dsigma += -(w_a - w_b)(v_a - v_b) dF_ab/dsigma  over faces ab
 //     (lambda_n, mu_n, dL/dtheta) = J_Phi^T (alpha w, mu_{n+1})
-// J_Phi^T is formed column block by column block with forward-mode dual
-// numbers through the same templated model code the forward kernels run
-// (model_tt2006.cuh), so the adjoint differentiates exactly the arithmetic of
-// the forward step.
+// J_Phi^T g is formed by one reverse sweep over the model's expression graph
+// (adj_cell): the gates' steady states and time constants, functions of V
+// alone, are differentiated by one forward-mode dual pass through the model
+// code the forward kernels run (tt2006_gate_rates), everything else by hand.
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "mb_internal.h"
@@ -20,133 +20,246 @@
 
 MB_NS_BEGIN
 
-// ---- dual numbers ---------------------------------------------------------------
+// ---- dual numbers (value and derivative with respect to one input) ---------------
 
 // value type T: double for the FP64 forward, float for the mixed one
-template <int K, typename T = double>
+template <typename T = double>
 struct Dual {
-    T v;
-    T d[K];
+    T v, d;
     __device__ __forceinline__ Dual() {}
-    __device__ __forceinline__ Dual(double x) : v((T)x) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) d[k] = T(0);
-    }
+    __device__ __forceinline__ Dual(double x) : v((T)x), d(T(0)) {}
+    __device__ __forceinline__ Dual(T x, T dx) : v(x), d(dx) {}
 };
 
-#define MB_DUAL_BIN(OP, VAL, DER)                                                                      \
-    template <int K, typename T>                                                                       \
-    __device__ __forceinline__ Dual<K, T> operator OP(const Dual<K, T> &a, const Dual<K, T> &b) {      \
-        Dual<K, T> r;                                                                                  \
-        r.v = VAL;                                                                                     \
-        _Pragma("unroll") for (int k = 0; k < K; ++k) r.d[k] = DER;                                    \
-        return r;                                                                                      \
-    }
-MB_DUAL_BIN(+, a.v + b.v, a.d[k] + b.d[k])
-MB_DUAL_BIN(-, a.v - b.v, a.d[k] - b.d[k])
-MB_DUAL_BIN(*, a.v * b.v, a.d[k] * b.v + a.v * b.d[k])
-MB_DUAL_BIN(/, a.v / b.v, (a.d[k] * b.v - a.v * b.d[k]) / (b.v * b.v))
-#undef MB_DUAL_BIN
-
-template <int K, typename T>
-__device__ __forceinline__ Dual<K, T> operator-(const Dual<K, T> &a) {
-    Dual<K, T> r;
-    r.v = -a.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = -a.d[k];
-    return r;
+#define MB_DUAL template <typename T> __device__ __forceinline__
+MB_DUAL Dual<T> operator+(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v + b.v, a.d + b.d); }
+MB_DUAL Dual<T> operator-(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v - b.v, a.d - b.d); }
+MB_DUAL Dual<T> operator*(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v * b.v, a.d * b.v + a.v * b.d); }
+MB_DUAL Dual<T> operator/(const Dual<T> &a, const Dual<T> &b) {
+    const T q = a.v / b.v;
+    return Dual<T>(q, (a.d - q * b.d) / b.v);
 }
-template <int K, typename T>
-__device__ __forceinline__ bool operator<(const Dual<K, T> &a, const Dual<K, T> &b) { return a.v < b.v; }
-template <int K, typename T>
-__device__ __forceinline__ bool operator>(const Dual<K, T> &a, const Dual<K, T> &b) { return a.v > b.v; }
-template <int K, typename T>
-__device__ __forceinline__ bool operator<=(const Dual<K, T> &a, const Dual<K, T> &b) { return a.v <= b.v; }
-template <int K, typename T>
-__device__ __forceinline__ bool operator>=(const Dual<K, T> &a, const Dual<K, T> &b) { return a.v >= b.v; }
-
-template <int K, typename T>
-__device__ __forceinline__ Dual<K, T> chain(const Dual<K, T> &a, T val, T der) {
-    Dual<K, T> r;
-    r.v = val;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = der * a.d[k];
-    return r;
-}
-// the value-type functions mexp / mexpm1 / mlog / msqrt of mb_math.cuh
-template <int K, typename T> __device__ __forceinline__ Dual<K, T> mexp(const Dual<K, T> &a) {
+MB_DUAL Dual<T> operator-(const Dual<T> &a) { return Dual<T>(-a.v, -a.d); }
+MB_DUAL bool operator<(const Dual<T> &a, const Dual<T> &b) { return a.v < b.v; }
+// the value-type functions mexp / msqrt of mb_math.cuh
+MB_DUAL Dual<T> mexp(const Dual<T> &a) {
     const T e = mexp(a.v);
-    return chain(a, e, e);
+    return Dual<T>(e, e * a.d);
 }
-template <int K, typename T> __device__ __forceinline__ Dual<K, T> mexpm1(const Dual<K, T> &a) {
-    return chain(a, mexpm1(a.v), mexp(a.v));
-}
-template <int K, typename T> __device__ __forceinline__ Dual<K, T> mlog(const Dual<K, T> &a) {
-    return chain(a, mlog(a.v), T(1) / a.v);
-}
-template <int K, typename T> __device__ __forceinline__ Dual<K, T> msqrt(const Dual<K, T> &a) {
+MB_DUAL Dual<T> msqrt(const Dual<T> &a) {
     const T s = msqrt(a.v);
-    return chain(a, s, T(0.5) / s);
+    return Dual<T>(s, T(0.5) / s * a.d);
 }
+#undef MB_DUAL
 
 // ---- ODE adjoint ----------------------------------------------------------------
 
 constexpr int ADJ_THREADS = 128;
 constexpr int ADJ_IN = TT_NEQ + 1;      // the 19 states and the gKr scaling
 
-// Column block [j0, j0 + K) of J_Phi, contracted with g: res[j] += sum_i g_i
-// d(out_i)/d(in_j).  Inputs 0..18 are the states (0 = V), input 19 the gKr
-// scaling.  T: the arithmetic of the forward step (double; float for the
-// mixed form, whose right-hand side is FP32); the contraction with g and the
-// results are FP64.
-template <int K, typename T = double>
-__device__ __forceinline__ void adj_block(int j0, const T (&y)[TT_NEQ], const TTScale<T> &sc, T stim, T dt,
-                                          const double (&g)[TT_NEQ], double (&res)[ADJ_IN]) {
-    using D = Dual<K, T>;
-    D yd[TT_NEQ];
-#pragma unroll
-    for (int s = 0; s < TT_NEQ; ++s) {
-        yd[s] = D(y[s]);
-#pragma unroll
-        for (int k = 0; k < K; ++k) yd[s].d[k] = (s == j0 + k) ? 1.0 : 0.0;
+// res = J_Phi^T g for one cell: Phi the Rush-Larsen sub-step of
+// tt2006_rhs at state y, res[j] = sum_i g_i d(out_i)/d(in_j) with inputs 0..18
+// the states (0 = V) and input 19 the gKr scaling.  T is the arithmetic of the
+// forward step (double; float for the mixed form, whose right-hand side is
+// FP32): model values and local derivatives are in T, the adjoint values they
+// are contracted with are FP64.
+//
+// What bounds it is the FP64 pipe and the latency of its chains (a 256 x 256
+// sheet is four warps per scheduler).  The sweep costs about three evaluations
+// of the model: 81 us per step on a 256 x 256 sheet in FP64 and 18 us on a
+// 97 x 131 sheet in FP32, against 1876 and 239 us for J column block by column
+// block with forward-mode duals (the model and two tangents, ten times).
+template <typename T>
+__device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> &sc, T dt, const double (&g)[TT_NEQ],
+                                         double (&res)[ADJ_IN]) {
+    const T V = y[TT_V];
+    const T Ca_i = y[TT_CAI], Ca_SR = y[TT_CASR], Ca_ss = y[TT_CASS], Rp = y[TT_RPRIME];
+    const T Na_i = y[TT_NAI], K_i = y[TT_KI];
+    const T R = T(8314.472), Tk = T(310.0), F = T(96485.3415f), RTF = (R * Tk) / F, FRT = F / (R * Tk);
+    const T Cm = T(0.185), V_c = T(0.016404), V_sr = T(0.001094f), V_ss = T(5.468e-05f);
+    const T Ko = T(5.4), Nao = T(140.0), Cao = T(2.0);
+    const double dtd = (double)dt;
+
+    // Euler states pass their own adjoint on; a = adjoint of the derivatives
+    double bV = g[TT_V], bcai = g[TT_CAI], bsr = g[TT_CASR], bss = g[TT_CASS], brp = g[TT_RPRIME];
+    double bnai = g[TT_NAI], bki = g[TT_KI];
+    const double aV = dtd * g[TT_V], aCai = dtd * g[TT_CAI], aSR = dtd * g[TT_CASR], aSS = dtd * g[TT_CASS];
+    const double aRp = dtd * g[TT_RPRIME], aNai = dtd * g[TT_NAI], aKi = dtd * g[TT_KI];
+
+    // buffers and their derivatives
+    const T K_buf_c = T(0.001f), K_buf_sr = T(0.3f), K_buf_ss = T(0.00025f);
+    const T qc = T(0.2f) * K_buf_c, qsr = T(10.0f) * K_buf_sr, qss = T(0.4f) * K_buf_ss;
+    const T cbc = Ca_i + K_buf_c, cbs = Ca_SR + K_buf_sr, cbss = Ca_ss + K_buf_ss;
+    const T Bc = T(1) / (T(1) + qc / (cbc * cbc)), Bsr = T(1) / (T(1) + qsr / (cbs * cbs));
+    const T Bss = T(1) / (T(1) + qss / (cbss * cbss));
+
+    // adjoints of the currents
+    const double kNa = (double)(Cm / (V_c * F)), kCa = 0.5 * kNa * (double)Bc;
+    const double kss = (double)(Cm / (T(2) * V_ss * F) * Bss);
+    const double bK = -aV - aKi * kNa;                  // IK1, Ito, IKr, IKs, IpK
+    const double bNa = -aV - aNai * kNa;                // INa, IbNa
+    const double bNaK = -aV - 3.0 * aNai * kNa + 2.0 * aKi * kNa;
+    const double bNaCa = -aV - 3.0 * aNai * kNa + 2.0 * aCai * kCa;
+    const double bCa = -aV - aCai * kCa;                // IbCa, IpCa
+    const double bCaL = -aV - aSS * kss;
+
+    // potassium currents
+    const T vek = V - RTF * mlog(Ko / K_i);
+    {
+        const T e1 = mexp(T(0.0002f) * (vek + T(100))), e2 = mexp(T(0.1f) * (vek - T(10))), e3 = mexp(T(-0.5f) * vek);
+        const T ea = mexp(T(0.06f) * (vek - T(200)));
+        const T d3 = T(1) / (T(1) + e3), da = T(1) / (T(1) + ea);
+        const T be = (T(3) * e1 + e2) * d3, al = T(0.1f) * da;
+        const T dbe = (T(3) * T(0.0002f) * e1 + T(0.1f) * e2) * d3 + T(0.5f) * e3 * d3 * be;
+        const T dal = -T(0.06f) * ea * da * al;
+        const T s = T(1) / (al + be), x = al * s;
+        const T dx = (dal * be - al * dbe) * s * s;
+        const T xr1 = y[TT_XR1], xr2 = y[TT_XR2], xs = y[TT_XS], r = y[TT_R], sg = y[TT_S];
+        const T gto = T(0.294), gpk = T(0.0146), gkr0 = T(0.153) * msqrt(Ko / T(5.4f)), gkr = gkr0 * sc.gKr;
+        const T ep = mexp((T(25) - V) / T(5.98f)), dp = T(1) / (T(1) + ep);
+        const double bvek = bK * (double)(T(5.405) * sc.gK1 * (x + vek * dx) + gto * r * sg + gkr * xr1 * xr2 + gpk * dp);
+        bV += bvek + bK * (double)(gpk * vek * ep / T(5.98f) * dp * dp);
+        bki += bvek * (double)(RTF / K_i);
+        res[TT_R] = bK * (double)(gto * sg * vek);
+        res[TT_S] = bK * (double)(gto * r * vek);
+        res[TT_XR1] = bK * (double)(gkr * xr2 * vek);
+        res[TT_XR2] = bK * (double)(gkr * xr1 * vek);
+        res[TT_NEQ] = bK * (double)(gkr0 * xr1 * xr2 * vek);
+        const T gks = T(0.098) * sc.gKs, ks = K_i + T(0.03) * Na_i;
+        const T vks = V - RTF * mlog((Ko + T(0.03) * Nao) / ks);
+        res[TT_XS] = bK * (double)(gks * T(2) * xs * vks);
+        const double t = bK * (double)(gks * xs * xs);
+        bV += t;
+        bki += t * (double)(RTF / ks);
+        bnai += t * (double)(RTF * T(0.03) / ks);
     }
-    TTScale<D> sd;
-    sd.gNa = D(sc.gNa);
-    sd.gKr = D(sc.gKr);
-    sd.gKs = D(sc.gKs);
-    sd.gCaL = D(sc.gCaL);
-    sd.gK1 = D(sc.gK1);
-#pragma unroll
-    for (int k = 0; k < K; ++k) sd.gKr.d[k] = (TT_NEQ == j0 + k) ? 1.0 : 0.0;
-    const D dtd(dt);
-    TTUpdate<D> u;
-    tt2006_rhs<D>(yd, D(stim), dtd, sd, u);
-    // the outputs of the sub-step, in the forms of k_tt2006_fp64
-    D out[TT_NEQ];
-    out[TT_V] = dtd * u.dV + yd[TT_V];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) out[1 + q] = u.gate[q];
-    out[TT_CAI] = dtd * u.dCai + yd[TT_CAI];
-    out[TT_CASR] = dtd * u.dCaSR + yd[TT_CASR];
-    out[TT_CASS] = dtd * u.dCaSS + yd[TT_CASS];
-    out[TT_RPRIME] = dtd * u.dRprime + yd[TT_RPRIME];
-    out[TT_NAI] = dtd * u.dNai + yd[TT_NAI];
-    out[TT_KI] = dtd * u.dKi + yd[TT_KI];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        if (j0 + k >= ADJ_IN) break;
-        double acc = 0.0;
-#pragma unroll
-        for (int i = 0; i < TT_NEQ; ++i) acc += g[i] * (double)out[i].d[k];
-        res[j0 + k] = acc;
+    // sodium currents
+    {
+        const T m = y[TT_M], h = y[TT_H], j = y[TT_J], gna = T(14.838) * sc.gNa;
+        const T vna = V - RTF * mlog(Nao / Na_i);
+        res[TT_M] = bNa * (double)(gna * T(3) * m * m * h * j * vna);
+        res[TT_H] = bNa * (double)(gna * (m * m * m) * j * vna);
+        res[TT_J] = bNa * (double)(gna * (m * m * m) * h * vna);
+        const double t = bNa * (double)(gna * (m * m * m) * h * j + T(0.00029));
+        bV += t;
+        bnai += t * (double)(RTF / Na_i);
     }
+    // sodium-potassium pump
+    {
+        const T e1 = mexp(T(-0.1f) * V * FRT), e2 = mexp(-V * FRT);
+        const T D = T(1) / (T(1) + T(0.1245f) * e1 + T(0.0353f) * e2);
+        const T P = T(2.724) * Ko / (Ko + T(1)), na = T(1) / (Na_i + T(40));
+        bnai += bNaK * (double)(P * T(40) * na * na * D);
+        bV += bNaK * (double)(P * Na_i * na * D * D * FRT * (T(0.1245f) * T(0.1f) * e1 + T(0.0353f) * e2));
+    }
+    // sodium-calcium exchanger
+    {
+        const T n = T(0.35), nm1 = n - T(1), na3 = Na_i * Na_i * Na_i, nao3 = Nao * Nao * Nao;
+        const T ep = mexp(n * V * FRT), em = mexp(nm1 * V * FRT);
+        const T C = (T(87.5) * T(87.5) * T(87.5) + nao3) * (T(1.38) + Cao);
+        const T D = T(1) / (T(1) + T(0.1) * em), k = T(1000) / C * D;
+        const T in = ep * na3 * Cao, out = em * nao3 * Ca_i * T(2.5);
+        bnai += bNaCa * (double)(k * T(3) * ep * (Na_i * Na_i) * Cao);
+        bcai -= bNaCa * (double)(k * em * nao3 * T(2.5));
+        bV += bNaCa * (double)(k * FRT * ((n * in - nm1 * out) - (in - out) * T(0.1) * nm1 * em * D));
+    }
+    // calcium background, pump and L-type currents
+    {
+        const double t = bCa * (double)T(0.000592);
+        bV += t;
+        bcai += t * (double)(T(0.5f) * RTF / Ca_i);
+        const T kp = Ca_i + T(0.0005);
+        bcai += bCa * (double)(T(0.1238) * T(0.0005) / (kp * kp));
+        const T v15 = V - T(15.0f), d = y[TT_D], f = y[TT_F], f2 = y[TT_F2], fc = y[TT_FCASS];
+        const T gca = T(3.98e-05) * sc.gCaL;
+        T G, GV, Gc;
+        if (V < T(15.0f - 1.0e-5f) || V > T(15.0f + 1.0e-5f)) {
+            const T k = T(2) * FRT, e = mexp(k * v15), im = T(1) / mexpm1(k * v15), c = T(4) * F * FRT;
+            const T A = T(0.25f) * Ca_ss * e - Cao;
+            G = c * v15 * A * im;
+            Gc = c * v15 * T(0.25f) * e * im;
+            GV = c * im * (A + v15 * k * e * (T(0.25f) * Ca_ss - A * im));
+        } else {                                        // the band's limit value does not depend on V
+            G = T(2) * F * (T(0.25f) * Ca_ss - Cao);
+            Gc = T(2) * F * T(0.25f);
+            GV = T(0);
+        }
+        const T gd = gca * d * f * f2 * fc;
+        bV += bCaL * (double)(gd * GV);
+        bss += bCaL * (double)(gd * Gc);
+        res[TT_D] = bCaL * (double)(gca * f * f2 * fc * G);
+        res[TT_F] = bCaL * (double)(gca * d * f2 * fc * G);
+        res[TT_F2] = bCaL * (double)(gca * d * f * fc * G);
+        res[TT_FCASS] = bCaL * (double)(gca * d * f * f2 * G);
+        // the buffered compartments: what multiplies Bc, Bsr and Bss
+        const T K_up2 = T(0.00025) * T(0.00025), V_rel = T(0.102), k3 = T(0.06), k4 = T(0.005f);
+        const T up = T(1) / (T(1) + K_up2 / (Ca_i * Ca_i)), i_up = T(0.006375) * up;
+        const T i_leak = T(0.00036f) * (Ca_SR - Ca_i), i_xfer = T(0.0038f) * (Ca_ss - Ca_i);
+        const T q2 = (T(1.5) / Ca_SR) * (T(1.5) / Ca_SR), iq = T(1) / (T(1) + q2);
+        const T kc = T(2.5) - T(1.5) * iq, k1 = T(0.15) / kc;
+        const T w = k1 * Ca_ss * Ca_ss, iw = T(1) / (k3 + w), O = w * Rp * iw, grad = Ca_SR - Ca_ss;
+        const T Irel = V_rel * O * grad;
+        const T IbCa = T(0.000592) * (V - T(0.5f) * RTF * mlog(Cao / Ca_i)), IpCa = T(0.1238) * Ca_i / kp;
+        const T nao3 = Nao * Nao * Nao, em = mexp((T(0.35) - T(1)) * V * FRT);
+        const T INaCa = T(1000) * (mexp(T(0.35) * V * FRT) * (Na_i * Na_i * Na_i) * Cao - em * nao3 * Ca_i * T(2.5)) /
+                        ((T(87.5) * T(87.5) * T(87.5) + nao3) * (T(1.38) + Cao) * (T(1) + T(0.1) * em));
+        const T sc_ = ((i_leak - i_up) * V_sr) / V_c + i_xfer - ((IbCa + IpCa - T(2) * INaCa) * Cm) / (T(2) * V_c * F);
+        const T ssr = i_up - (Irel + i_leak);
+        const T sss = (-gd * G * Cm) / (T(2) * V_ss * F) + (Irel * V_sr) / V_ss - (i_xfer * V_c) / V_ss;
+        bcai += aCai * (double)(sc_ * Bc * Bc * T(2) * qc / (cbc * cbc * cbc));
+        bsr += aSR * (double)(ssr * Bsr * Bsr * T(2) * qsr / (cbs * cbs * cbs));
+        bss += aSS * (double)(sss * Bss * Bss * T(2) * qss / (cbss * cbss * cbss));
+        // fluxes
+        const double uc = aCai * (double)Bc, us = aSR * (double)Bsr, uss = aSS * (double)Bss;
+        const double vr = (double)(V_sr / V_c);
+        const double bup = us - uc * vr, bleak = uc * vr - us, bx = uc - uss * (double)(V_c / V_ss);
+        const double brel = uss * (double)(V_sr / V_ss) - us;
+        bcai += bup * (double)(T(0.006375) * up * up * T(2) * K_up2 / (Ca_i * Ca_i * Ca_i));
+        bsr += bleak * (double)T(0.00036f);
+        bcai -= bleak * (double)T(0.00036f);
+        bss += bx * (double)T(0.0038f);
+        bcai -= bx * (double)T(0.0038f);
+        // release: O and R'
+        const double bO = brel * (double)(V_rel * grad);
+        bsr += brel * (double)(V_rel * O);
+        bss -= brel * (double)(V_rel * O);
+        const double bw = bO * (double)(Rp * k3 * iw * iw);
+        const T k2 = T(0.045f) * kc;
+        brp += bO * (double)(w * iw) - aRp * (double)(k2 * Ca_ss + k4);
+        bss += bw * (double)(T(2) * k1 * Ca_ss) - aRp * (double)(k2 * Rp);
+        const double bkc = -aRp * (double)(T(0.045f) * Ca_ss * Rp) - bw * (double)(w / kc);
+        bsr -= bkc * (double)(T(1.5) * T(2) * q2 * iq * iq / Ca_SR);
+    }
+    // gates: inf + (y - inf) exp(-dt / tau)
+    {
+        Dual<T> inf[12], tau[12];
+        tt2006_gate_rates<Dual<T>>(Dual<T>(V, T(1)), Dual<T>(Ca_ss, T(0)), inf, tau);
+        // fCass follows Ca_ss: inf = 0.6 / (1 + c^2) + 0.4, tau = 80 / (1 + c^2) + 2, c = Ca_ss / 0.05
+        const T c = Ca_ss / T(0.05f), ic = T(1) / (T(1) + c * c), dc = -T(2) * c / T(0.05f) * ic * ic;
+        inf[9].d = T(0.6f) * dc;
+        tau[9].d = T(80.0f) * dc;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const T E = mexp(-dt / tau[k].v);
+            const double b = g[1 + k] * (double)((T(1) - E) * inf[k].d + (y[1 + k] - inf[k].v) * E *
+                                                 (dt * tau[k].d / (tau[k].v * tau[k].v)));
+            if (k == 9) bss += b;
+            else bV += b;
+            res[1 + k] += g[1 + k] * (double)E;
+        }
+    }
+    res[TT_V] = bV;
+    res[TT_CAI] = bcai;
+    res[TT_CASR] = bsr;
+    res[TT_CASS] = bss;
+    res[TT_RPRIME] = brp;
+    res[TT_NAI] = bnai;
+    res[TT_KI] = bki;
 }
 
 // Per compact cell t: y = (v_n, s_n) from a snapshot, g = (alpha w, mu_in);
 // writes lambda_n (grid), mu_out (state rows 1..18) and adds dL/dgKr.
-template <int K>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl_n,
-                                                            const double *__restrict__ v_n,
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006(mb_ode_dev o, const double *__restrict__ v_n,
                                                             const double *__restrict__ sv_n,
                                                             const double *__restrict__ w, double alpha,
                                                             const double *__restrict__ mu_in, double *mu_out,
@@ -163,10 +276,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006(mb_ode_dev o, const 
         y[s] = sv_n[s * ld + t];
         gi[s] = mu_in[s * ld + t];
     }
-    const double stim = cell_stim(o, ctrl_n, t);
     const TTScale<double> sc = load_tt_scale<double>(o, t);
     double res[ADJ_IN];
-    for (int j0 = 0; j0 < ADJ_IN; j0 += K) adj_block<K>(j0, y, sc, stim, o.dt, gi, res);
+    adj_cell<double>(y, sc, o.dt, gi, res);
     lam_out[g] = res[0];
 #pragma unroll
     for (int s = 1; s < TT_NEQ; ++s) mu_out[s * ld + t] = res[s];
@@ -175,11 +287,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006(mb_ode_dev o, const 
 
 // The same for the mixed forward (k_tt2006_mixed): the state from the mixed
 // rows of the snapshot (FP64 rows 1..5 = Ca_i, Ca_SR, Ca_ss, Na_i, K_i; FP32
-// rows 0..11 = the gates, row 12 = R'), the Jacobian in FP32 dual numbers
-// through the same model code, contracted and accumulated in FP64.
-template <int K>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006_mixed(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl_n,
-                                                                  const double *__restrict__ v_n,
+// rows 0..11 = the gates, row 12 = R'), the local derivatives in FP32,
+// contracted and accumulated in FP64.
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006_mixed(mb_ode_dev o, const double *__restrict__ v_n,
                                                                   const double *__restrict__ sv64_n,
                                                                   const float *__restrict__ sv32_n,
                                                                   const double *__restrict__ w, double alpha,
@@ -203,10 +313,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006_mixed(mb_ode_dev o, 
     gi[0] = alpha * w[g];
 #pragma unroll
     for (int s = 1; s < TT_NEQ; ++s) gi[s] = mu_in[s * ld + t];
-    const float stim = (float)cell_stim(o, ctrl_n, t);
     const TTScale<float> sc = load_tt_scale<float>(o, t);
     double res[ADJ_IN];
-    for (int j0 = 0; j0 < ADJ_IN; j0 += K) adj_block<K, float>(j0, y, sc, stim, (float)o.dt, gi, res);
+    adj_cell<float>(y, sc, (float)o.dt, gi, res);
     lam_out[g] = res[0];
 #pragma unroll
     for (int s = 1; s < TT_NEQ; ++s) mu_out[s * ld + t] = res[s];
@@ -277,19 +386,19 @@ MB_NS_END
 
 using namespace mb;
 
-extern "C" int mbk_adj_tt2006(const mb_ode_dev *o, const mb_ctrl *ctrl_n, const double *v_n, const double *sv_n,
+extern "C" int mbk_adj_tt2006(const mb_ode_dev *o, const double *v_n, const double *sv_n,
                               const double *w, double alpha, const double *mu_in, double *mu_out, double *lam_out,
                               double *gth, cudaStream_t s) {
     const unsigned blocks = (o->n + ADJ_THREADS - 1) / ADJ_THREADS;
-    k_adj_tt2006<2><<<blocks, ADJ_THREADS, 0, s>>>(*o, ctrl_n, v_n, sv_n, w, alpha, mu_in, mu_out, lam_out, gth);
+    k_adj_tt2006<<<blocks, ADJ_THREADS, 0, s>>>(*o, v_n, sv_n, w, alpha, mu_in, mu_out, lam_out, gth);
     return (int)cudaGetLastError();
 }
 
-extern "C" int mbk_adj_tt2006_mixed(const mb_ode_dev *o, const mb_ctrl *ctrl_n, const double *v_n,
+extern "C" int mbk_adj_tt2006_mixed(const mb_ode_dev *o, const double *v_n,
                                     const double *sv64_n, const float *sv32_n, const double *w, double alpha,
                                     const double *mu_in, double *mu_out, double *lam_out, double *gth, cudaStream_t s) {
     const unsigned blocks = (o->n + ADJ_THREADS - 1) / ADJ_THREADS;
-    k_adj_tt2006_mixed<2><<<blocks, ADJ_THREADS, 0, s>>>(*o, ctrl_n, v_n, sv64_n, sv32_n, w, alpha, mu_in, mu_out,
+    k_adj_tt2006_mixed<<<blocks, ADJ_THREADS, 0, s>>>(*o, v_n, sv64_n, sv32_n, w, alpha, mu_in, mu_out,
                                                         lam_out, gth);
     return (int)cudaGetLastError();
 }

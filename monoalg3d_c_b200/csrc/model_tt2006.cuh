@@ -50,6 +50,80 @@ struct TTUpdate {
     T dCai, dCaSR, dCaSS, dRprime, dNai, dKi;
 };
 
+// Steady states and time constants of gates 1..12 (state order): functions of V,
+// for fCass of Ca_ss.
+template <typename T>
+__device__ __forceinline__ void tt2006_gate_rates(const T V, const T Ca_ss, T (&inf)[12], T (&tau)[12]) {
+    // gating variables: steady states and time constants
+    const T xr1_inf = T(1.0f) / (T(1.0f) + mexp((T(-26.0f) - V) / T(7.0f)));
+    const T tau_xr1 = (T(450.0f) / (T(1.0f) + mexp((T(-45.0f) - V) / T(10.0f)))) *
+                      (T(6.0f) / (T(1.0f) + mexp((V + T(30.0f)) / T(11.5f))));
+    const T xr2_inf = T(1.0f) / (T(1.0f) + mexp((V + T(88.0f)) / T(24.0f)));
+    const T tau_xr2 = (T(3.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(20.0f)))) *
+                      (T(1.12f) / (T(1.0f) + mexp((V - T(60.0f)) / T(20.0f))));
+    const T xs_inf = T(1.0f) / (T(1.0f) + mexp((T(-5.0f) - V) / T(14.0f)));
+    const T tau_xs = ((T(1400.0f) / msqrt(T(1.0f) + mexp((T(5.0f) - V) / T(6.0f)))) *
+                      (T(1.0f) / (T(1.0f) + mexp((V - T(35.0f)) / T(15.0f))))) + T(80.0f);
+
+    const T em = T(1.0f) + mexp((T(-56.86f) - V) / T(9.03f));
+    const T m_inf = T(1.0f) / (em * em);
+    const T tau_m = (T(1.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(5.0f)))) *
+                    ((T(0.1f) / (T(1.0f) + mexp((V + T(35.0f)) / T(5.0f)))) +
+                     (T(0.1f) / (T(1.0f) + mexp((V - T(50.0f)) / T(200.0f)))));
+
+    const T eh = T(1.0f) + mexp((V + T(71.55f)) / T(7.43f));
+    const T h_inf = T(1.0f) / (eh * eh);
+    const T j_inf = h_inf;
+    T alpha_h, beta_h, alpha_j, beta_j;
+    if (V < T(-40.0f)) {
+        alpha_h = T(0.057f) * mexp((-(V + T(80.0f))) / T(6.8f));
+        beta_h = (T(2.7f) * mexp(T(0.079f) * V)) + (T(310000.0f) * mexp(T(0.3485f) * V));
+        alpha_j = ((((T(-25428.0f)) * mexp(T(0.2444f) * V)) - (T(6.948e-06f) * mexp(T(-0.04391f) * V))) *
+                   (V + T(37.78f))) / (T(1.0f) + mexp(T(0.311f) * (V + T(79.23f))));
+        beta_j = (T(0.02424f) * mexp(T(-0.01052f) * V)) / (T(1.0f) + mexp(T(-0.1378f) * (V + T(40.14f))));
+    } else {
+        alpha_h = T(0.0f);
+        beta_h = T(0.77f) / (T(0.13f) * (T(1.0f) + mexp((V + T(10.66f)) / T(-11.1f))));
+        alpha_j = T(0.0f);
+        beta_j = (T(0.6f) * mexp(T(0.057f) * V)) / (T(1.0f) + mexp(T(-0.1f) * (V + T(32.0f))));
+    }
+    const T tau_h = T(1.0f) / (alpha_h + beta_h);
+    const T tau_j = T(1.0f) / (alpha_j + beta_j);
+
+    const T d_inf = T(1.0f) / (T(1.0f) + mexp((T(-8.0f) - V) / T(7.5f)));
+    const T tau_d = ((T(1.4f) / (T(1.0f) + mexp((T(-35.0f) - V) / T(13.0f)))) + T(0.25f)) *
+                        (T(1.4f) / (T(1.0f) + mexp((V + T(5.0f)) / T(5.0f)))) +
+                    (T(1.0f) / (T(1.0f) + mexp((T(50.0f) - V) / T(20.0f))));
+
+    const T e30 = mexp((V + T(30.0f)) / T(10.0f));
+    const T v27 = V + T(27.0f);
+    const T f_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(7.0f)));
+    const T tau_f = (T(1102.5f) * mexp((-(v27 * v27)) / T(225.0f))) +
+                    (T(200.0f) / (T(1.0f) + mexp((T(13.0f) - V) / T(10.0f)))) +
+                    (T(180.0f) / (T(1.0f) + e30)) + T(20.0f);
+    const T f2_inf = (T(0.67f) / (T(1.0f) + mexp((V + T(35.0f)) / T(7.0f)))) + T(0.33f);
+    const T tau_f2 = (T(562.0f) * mexp((-(v27 * v27)) / T(240.0f))) +
+                     (T(31.0f) / (T(1.0f) + mexp((T(25.0f) - V) / T(10.0f)))) +
+                     (T(80.0f) / (T(1.0f) + e30));
+
+    const T cr = Ca_ss / T(0.05f);
+    const T fCass_inf = (T(0.6f) / (T(1.0f) + cr * cr)) + T(0.4f);
+    const T tau_fCass = (T(80.0f) / (T(1.0f) + cr * cr)) + T(2.0f);
+
+    const T s_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(5.0f)));
+    const T v45 = V + T(45.0f);
+    const T tau_s = (T(85.0f) * mexp((-(v45 * v45)) / T(320.0f))) +
+                    (T(5.0f) / (T(1.0f) + mexp((V - T(20.0f)) / T(5.0f)))) + T(3.0f);
+    const T r_inf = T(1.0f) / (T(1.0f) + mexp((T(20.0f) - V) / T(6.0f)));
+    const T v40 = V + T(40.0f);
+    const T tau_r = (T(9.5f) * mexp((-(v40 * v40)) / T(1800.0f))) + T(0.8f);
+
+    inf[0] = xr1_inf; inf[1] = xr2_inf; inf[2] = xs_inf; inf[3] = m_inf; inf[4] = h_inf; inf[5] = j_inf;
+    inf[6] = d_inf; inf[7] = f_inf; inf[8] = f2_inf; inf[9] = fCass_inf; inf[10] = s_inf; inf[11] = r_inf;
+    tau[0] = tau_xr1; tau[1] = tau_xr2; tau[2] = tau_xs; tau[3] = tau_m; tau[4] = tau_h; tau[5] = tau_j;
+    tau[6] = tau_d; tau[7] = tau_f; tau[8] = tau_f2; tau[9] = tau_fCass; tau[10] = tau_s; tau[11] = tau_r;
+}
+
 // y: the 19 state values (in T), stim: merged stimulus current.
 template <typename T>
 __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTScale<T> &sc,
@@ -124,69 +198,8 @@ __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTSca
                      (T(1.0f) + (K_sat * e_gm1)));
     (void)FRT;
 
-    // gating variables: steady states and time constants
-    const T xr1_inf = T(1.0f) / (T(1.0f) + mexp((T(-26.0f) - V) / T(7.0f)));
-    const T tau_xr1 = (T(450.0f) / (T(1.0f) + mexp((T(-45.0f) - V) / T(10.0f)))) *
-                      (T(6.0f) / (T(1.0f) + mexp((V + T(30.0f)) / T(11.5f))));
-    const T xr2_inf = T(1.0f) / (T(1.0f) + mexp((V + T(88.0f)) / T(24.0f)));
-    const T tau_xr2 = (T(3.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(20.0f)))) *
-                      (T(1.12f) / (T(1.0f) + mexp((V - T(60.0f)) / T(20.0f))));
-    const T xs_inf = T(1.0f) / (T(1.0f) + mexp((T(-5.0f) - V) / T(14.0f)));
-    const T tau_xs = ((T(1400.0f) / msqrt(T(1.0f) + mexp((T(5.0f) - V) / T(6.0f)))) *
-                      (T(1.0f) / (T(1.0f) + mexp((V - T(35.0f)) / T(15.0f))))) + T(80.0f);
-
-    const T em = T(1.0f) + mexp((T(-56.86f) - V) / T(9.03f));
-    const T m_inf = T(1.0f) / (em * em);
-    const T tau_m = (T(1.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(5.0f)))) *
-                    ((T(0.1f) / (T(1.0f) + mexp((V + T(35.0f)) / T(5.0f)))) +
-                     (T(0.1f) / (T(1.0f) + mexp((V - T(50.0f)) / T(200.0f)))));
-
-    const T eh = T(1.0f) + mexp((V + T(71.55f)) / T(7.43f));
-    const T h_inf = T(1.0f) / (eh * eh);
-    const T j_inf = h_inf;
-    T alpha_h, beta_h, alpha_j, beta_j;
-    if (V < T(-40.0f)) {
-        alpha_h = T(0.057f) * mexp((-(V + T(80.0f))) / T(6.8f));
-        beta_h = (T(2.7f) * mexp(T(0.079f) * V)) + (T(310000.0f) * mexp(T(0.3485f) * V));
-        alpha_j = ((((T(-25428.0f)) * mexp(T(0.2444f) * V)) - (T(6.948e-06f) * mexp(T(-0.04391f) * V))) *
-                   (V + T(37.78f))) / (T(1.0f) + mexp(T(0.311f) * (V + T(79.23f))));
-        beta_j = (T(0.02424f) * mexp(T(-0.01052f) * V)) / (T(1.0f) + mexp(T(-0.1378f) * (V + T(40.14f))));
-    } else {
-        alpha_h = T(0.0f);
-        beta_h = T(0.77f) / (T(0.13f) * (T(1.0f) + mexp((V + T(10.66f)) / T(-11.1f))));
-        alpha_j = T(0.0f);
-        beta_j = (T(0.6f) * mexp(T(0.057f) * V)) / (T(1.0f) + mexp(T(-0.1f) * (V + T(32.0f))));
-    }
-    const T tau_h = T(1.0f) / (alpha_h + beta_h);
-    const T tau_j = T(1.0f) / (alpha_j + beta_j);
-
-    const T d_inf = T(1.0f) / (T(1.0f) + mexp((T(-8.0f) - V) / T(7.5f)));
-    const T tau_d = ((T(1.4f) / (T(1.0f) + mexp((T(-35.0f) - V) / T(13.0f)))) + T(0.25f)) *
-                        (T(1.4f) / (T(1.0f) + mexp((V + T(5.0f)) / T(5.0f)))) +
-                    (T(1.0f) / (T(1.0f) + mexp((T(50.0f) - V) / T(20.0f))));
-
-    const T e30 = mexp((V + T(30.0f)) / T(10.0f));
-    const T v27 = V + T(27.0f);
-    const T f_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(7.0f)));
-    const T tau_f = (T(1102.5f) * mexp((-(v27 * v27)) / T(225.0f))) +
-                    (T(200.0f) / (T(1.0f) + mexp((T(13.0f) - V) / T(10.0f)))) +
-                    (T(180.0f) / (T(1.0f) + e30)) + T(20.0f);
-    const T f2_inf = (T(0.67f) / (T(1.0f) + mexp((V + T(35.0f)) / T(7.0f)))) + T(0.33f);
-    const T tau_f2 = (T(562.0f) * mexp((-(v27 * v27)) / T(240.0f))) +
-                     (T(31.0f) / (T(1.0f) + mexp((T(25.0f) - V) / T(10.0f)))) +
-                     (T(80.0f) / (T(1.0f) + e30));
-
-    const T cr = Ca_ss / T(0.05f);
-    const T fCass_inf = (T(0.6f) / (T(1.0f) + cr * cr)) + T(0.4f);
-    const T tau_fCass = (T(80.0f) / (T(1.0f) + cr * cr)) + T(2.0f);
-
-    const T s_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(5.0f)));
-    const T v45 = V + T(45.0f);
-    const T tau_s = (T(85.0f) * mexp((-(v45 * v45)) / T(320.0f))) +
-                    (T(5.0f) / (T(1.0f) + mexp((V - T(20.0f)) / T(5.0f)))) + T(3.0f);
-    const T r_inf = T(1.0f) / (T(1.0f) + mexp((T(20.0f) - V) / T(6.0f)));
-    const T v40 = V + T(40.0f);
-    const T tau_r = (T(9.5f) * mexp((-(v40 * v40)) / T(1800.0f))) + T(0.8f);
+    T inf[12], tau[12];
+    tt2006_gate_rates<T>(V, Ca_ss, inf, tau);
 
     // calcium dynamics
     const T ecs = EC / Ca_SR;
@@ -224,18 +237,8 @@ __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTSca
     u.dKi = ((-((IK1 + Ito + IKr + IKs + IpK + stim) - (T(2.0f) * INaK))) / (V_c * F)) * Cm;
 
     // Rush-Larsen gate updates
-    u.gate[0] = xr1_inf + (Xr1 - xr1_inf) * mexp(-dt / tau_xr1);
-    u.gate[1] = xr2_inf + (Xr2 - xr2_inf) * mexp(-dt / tau_xr2);
-    u.gate[2] = xs_inf + (Xs - xs_inf) * mexp(-dt / tau_xs);
-    u.gate[3] = m_inf + (m - m_inf) * mexp(-dt / tau_m);
-    u.gate[4] = h_inf + (h - h_inf) * mexp(-dt / tau_h);
-    u.gate[5] = j_inf + (j - j_inf) * mexp(-dt / tau_j);
-    u.gate[6] = d_inf + (d - d_inf) * mexp(-dt / tau_d);
-    u.gate[7] = f_inf + (f - f_inf) * mexp(-dt / tau_f);
-    u.gate[8] = f2_inf + (f2 - f2_inf) * mexp(-dt / tau_f2);
-    u.gate[9] = fCass_inf + (fCass - fCass_inf) * mexp(-dt / tau_fCass);
-    u.gate[10] = s_inf + (s - s_inf) * mexp(-dt / tau_s);
-    u.gate[11] = r_inf + (r - r_inf) * mexp(-dt / tau_r);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) u.gate[k] = inf[k] + (y[TT_XR1 + k] - inf[k]) * mexp(-dt / tau[k]);
 }
 
 MB_NS_END
