@@ -421,8 +421,8 @@ int mb_monodomain_time_steps_host_async(mb_monodomain *m, int n, const double *s
                                         double *v0, double *v1, double *ms);
 
 /* Launch choices made at creation by timing: the ODE kernel's variant
- * (0..5 = one-cell-per-thread launches with at least 1..6 resident 128-thread
- * blocks per SM, 6..9 = staged persistent launches with at least 1..4), the
+ * (0..5 = one-cell-per-thread launches of 128-thread blocks, in the order of
+ * their occupancy, 6..9 = staged persistent launches), the
  * CG grid size and the CG kernel (-1 = graph of separate kernels, 0..n-1 =
  * launch shape of the flat persistent kernel, n = mb_cg_launch_shapes --
  * the first half with a contiguous range of cells per block, the second the

@@ -35,20 +35,24 @@ struct Dual {
 MB_DUAL Dual<T> operator+(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v + b.v, a.d + b.d); }
 MB_DUAL Dual<T> operator-(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v - b.v, a.d - b.d); }
 MB_DUAL Dual<T> operator*(const Dual<T> &a, const Dual<T> &b) { return Dual<T>(a.v * b.v, a.d * b.v + a.v * b.d); }
-MB_DUAL Dual<T> operator/(const Dual<T> &a, const Dual<T> &b) {
-    const T q = a.v / b.v;
-    return Dual<T>(q, (a.d - q * b.d) / b.v);
-}
 MB_DUAL Dual<T> operator-(const Dual<T> &a) { return Dual<T>(-a.v, -a.d); }
 MB_DUAL bool operator<(const Dual<T> &a, const Dual<T> &b) { return a.v < b.v; }
-// the value-type functions mexp / msqrt of mb_math.cuh
+// the value-type functions of mb_math.cuh
+MB_DUAL Dual<T> mrcp(const Dual<T> &a) {
+    const T y = mrcp(a.v);
+    return Dual<T>(y, -y * y * a.d);
+}
+MB_DUAL Dual<T> mdiv(const Dual<T> &a, const Dual<T> &b) {
+    const T q = mdiv(a.v, b.v);
+    return Dual<T>(q, (a.d - q * b.d) * mrcp(b.v));
+}
 MB_DUAL Dual<T> mexp(const Dual<T> &a) {
     const T e = mexp(a.v);
     return Dual<T>(e, e * a.d);
 }
 MB_DUAL Dual<T> msqrt(const Dual<T> &a) {
     const T s = msqrt(a.v);
-    return Dual<T>(s, T(0.5) / s * a.d);
+    return Dual<T>(s, mdiv(T(0.5), s) * a.d);
 }
 #undef MB_DUAL
 
@@ -90,8 +94,8 @@ __device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> 
     const T K_buf_c = T(0.001f), K_buf_sr = T(0.3f), K_buf_ss = T(0.00025f);
     const T qc = T(0.2f) * K_buf_c, qsr = T(10.0f) * K_buf_sr, qss = T(0.4f) * K_buf_ss;
     const T cbc = Ca_i + K_buf_c, cbs = Ca_SR + K_buf_sr, cbss = Ca_ss + K_buf_ss;
-    const T Bc = T(1) / (T(1) + qc / (cbc * cbc)), Bsr = T(1) / (T(1) + qsr / (cbs * cbs));
-    const T Bss = T(1) / (T(1) + qss / (cbss * cbss));
+    const T ic = mrcp(cbc * cbc + qc), isr = mrcp(cbs * cbs + qsr), iss = mrcp(cbss * cbss + qss);
+    const T Bc = cbc * cbc * ic, Bsr = cbs * cbs * isr, Bss = cbss * cbss * iss;
 
     // adjoints of the currents
     const double kNa = (double)(Cm / (V_c * F)), kCa = 0.5 * kNa * (double)Bc;
@@ -104,61 +108,63 @@ __device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> 
     const double bCaL = -aV - aSS * kss;
 
     // potassium currents
-    const T vek = V - RTF * mlog(Ko / K_i);
+    const T vek = V - RTF * mlog(mdiv(Ko, K_i));
     {
         const T e1 = mexp(T(0.0002f) * (vek + T(100))), e2 = mexp(T(0.1f) * (vek - T(10))), e3 = mexp(T(-0.5f) * vek);
         const T ea = mexp(T(0.06f) * (vek - T(200)));
-        const T d3 = T(1) / (T(1) + e3), da = T(1) / (T(1) + ea);
+        const T d3 = mrcp(T(1) + e3), da = mrcp(T(1) + ea);
         const T be = (T(3) * e1 + e2) * d3, al = T(0.1f) * da;
         const T dbe = (T(3) * T(0.0002f) * e1 + T(0.1f) * e2) * d3 + T(0.5f) * e3 * d3 * be;
         const T dal = -T(0.06f) * ea * da * al;
-        const T s = T(1) / (al + be), x = al * s;
+        const T s = mrcp(al + be), x = al * s;
         const T dx = (dal * be - al * dbe) * s * s;
         const T xr1 = y[TT_XR1], xr2 = y[TT_XR2], xs = y[TT_XS], r = y[TT_R], sg = y[TT_S];
-        const T gto = T(0.294), gpk = T(0.0146), gkr0 = T(0.153) * msqrt(Ko / T(5.4f)), gkr = gkr0 * sc.gKr;
-        const T ep = mexp((T(25) - V) / T(5.98f)), dp = T(1) / (T(1) + ep);
+        const T gto = T(0.294), gpk = T(0.0146), gkr0 = T(0.153) * T(TT_SQRT_KO), gkr = gkr0 * sc.gKr;
+        const T ep = mexp(MB_OVER(T(25) - V, (double)5.98f)), dp = mrcp(T(1) + ep);
         const double bvek = bK * (double)(T(5.405) * sc.gK1 * (x + vek * dx) + gto * r * sg + gkr * xr1 * xr2 + gpk * dp);
-        bV += bvek + bK * (double)(gpk * vek * ep / T(5.98f) * dp * dp);
-        bki += bvek * (double)(RTF / K_i);
+        bV += bvek + bK * (double)(gpk * vek * MB_OVER(ep, (double)5.98f) * dp * dp);
+        bki += bvek * (double)mdiv(RTF, K_i);
         res[TT_R] = bK * (double)(gto * sg * vek);
         res[TT_S] = bK * (double)(gto * r * vek);
         res[TT_XR1] = bK * (double)(gkr * xr2 * vek);
         res[TT_XR2] = bK * (double)(gkr * xr1 * vek);
         res[TT_NEQ] = bK * (double)(gkr0 * xr1 * xr2 * vek);
         const T gks = T(0.098) * sc.gKs, ks = K_i + T(0.03) * Na_i;
-        const T vks = V - RTF * mlog((Ko + T(0.03) * Nao) / ks);
+        const T iks = mrcp(ks), vks = V - RTF * mlog(mdiv(Ko + T(0.03) * Nao, ks));
         res[TT_XS] = bK * (double)(gks * T(2) * xs * vks);
         const double t = bK * (double)(gks * xs * xs);
         bV += t;
-        bki += t * (double)(RTF / ks);
-        bnai += t * (double)(RTF * T(0.03) / ks);
+        bki += t * (double)(RTF * iks);
+        bnai += t * (double)(RTF * T(0.03) * iks);
     }
     // sodium currents
     {
         const T m = y[TT_M], h = y[TT_H], j = y[TT_J], gna = T(14.838) * sc.gNa;
-        const T vna = V - RTF * mlog(Nao / Na_i);
+        const T vna = V - RTF * mlog(mdiv(Nao, Na_i));
         res[TT_M] = bNa * (double)(gna * T(3) * m * m * h * j * vna);
         res[TT_H] = bNa * (double)(gna * (m * m * m) * j * vna);
         res[TT_J] = bNa * (double)(gna * (m * m * m) * h * vna);
         const double t = bNa * (double)(gna * (m * m * m) * h * j + T(0.00029));
         bV += t;
-        bnai += t * (double)(RTF / Na_i);
+        bnai += t * (double)mdiv(RTF, Na_i);
     }
     // sodium-potassium pump
     {
         const T e1 = mexp(T(-0.1f) * V * FRT), e2 = mexp(-V * FRT);
-        const T D = T(1) / (T(1) + T(0.1245f) * e1 + T(0.0353f) * e2);
-        const T P = T(2.724) * Ko / (Ko + T(1)), na = T(1) / (Na_i + T(40));
+        const T D = mrcp(T(1) + T(0.1245f) * e1 + T(0.0353f) * e2);
+        const T P = T(2.724) * Ko / (Ko + T(1)), na = mrcp(Na_i + T(40));
         bnai += bNaK * (double)(P * T(40) * na * na * D);
         bV += bNaK * (double)(P * Na_i * na * D * D * FRT * (T(0.1245f) * T(0.1f) * e1 + T(0.0353f) * e2));
     }
     // sodium-calcium exchanger
+    T INaCa;
     {
         const T n = T(0.35), nm1 = n - T(1), na3 = Na_i * Na_i * Na_i, nao3 = Nao * Nao * Nao;
         const T ep = mexp(n * V * FRT), em = mexp(nm1 * V * FRT);
         const T C = (T(87.5) * T(87.5) * T(87.5) + nao3) * (T(1.38) + Cao);
-        const T D = T(1) / (T(1) + T(0.1) * em), k = T(1000) / C * D;
+        const T D = mrcp(T(1) + T(0.1) * em), k = T(1000) / C * D;
         const T in = ep * na3 * Cao, out = em * nao3 * Ca_i * T(2.5);
+        INaCa = k * (in - out);
         bnai += bNaCa * (double)(k * T(3) * ep * (Na_i * Na_i) * Cao);
         bcai -= bNaCa * (double)(k * em * nao3 * T(2.5));
         bV += bNaCa * (double)(k * FRT * ((n * in - nm1 * out) - (in - out) * T(0.1) * nm1 * em * D));
@@ -167,14 +173,14 @@ __device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> 
     {
         const double t = bCa * (double)T(0.000592);
         bV += t;
-        bcai += t * (double)(T(0.5f) * RTF / Ca_i);
-        const T kp = Ca_i + T(0.0005);
-        bcai += bCa * (double)(T(0.1238) * T(0.0005) / (kp * kp));
+        bcai += t * (double)mdiv(T(0.5f) * RTF, Ca_i);
+        const T kp = mrcp(Ca_i + T(0.0005));
+        bcai += bCa * (double)(T(0.1238) * T(0.0005) * kp * kp);
         const T v15 = V - T(15.0f), d = y[TT_D], f = y[TT_F], f2 = y[TT_F2], fc = y[TT_FCASS];
         const T gca = T(3.98e-05) * sc.gCaL;
         T G, GV, Gc;
         if (V < T(15.0f - 1.0e-5f) || V > T(15.0f + 1.0e-5f)) {
-            const T k = T(2) * FRT, e = mexp(k * v15), im = T(1) / mexpm1(k * v15), c = T(4) * F * FRT;
+            const T k = T(2) * FRT, e = mexp(k * v15), im = mrcp(mexpm1(k * v15)), c = T(4) * F * FRT;
             const T A = T(0.25f) * Ca_ss * e - Cao;
             G = c * v15 * A * im;
             Gc = c * v15 * T(0.25f) * e * im;
@@ -193,28 +199,25 @@ __device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> 
         res[TT_FCASS] = bCaL * (double)(gca * d * f * f2 * G);
         // the buffered compartments: what multiplies Bc, Bsr and Bss
         const T K_up2 = T(0.00025) * T(0.00025), V_rel = T(0.102), k3 = T(0.06), k4 = T(0.005f);
-        const T up = T(1) / (T(1) + K_up2 / (Ca_i * Ca_i)), i_up = T(0.006375) * up;
+        const T iu = mrcp(Ca_i * Ca_i + K_up2), i_up = T(0.006375) * (Ca_i * Ca_i * iu);
         const T i_leak = T(0.00036f) * (Ca_SR - Ca_i), i_xfer = T(0.0038f) * (Ca_ss - Ca_i);
-        const T q2 = (T(1.5) / Ca_SR) * (T(1.5) / Ca_SR), iq = T(1) / (T(1) + q2);
-        const T kc = T(2.5) - T(1.5) * iq, k1 = T(0.15) / kc;
-        const T w = k1 * Ca_ss * Ca_ss, iw = T(1) / (k3 + w), O = w * Rp * iw, grad = Ca_SR - Ca_ss;
+        const T iq = mrcp(Ca_SR * Ca_SR + T(1.5) * T(1.5));
+        const T kc = T(2.5) - T(1.5) * (Ca_SR * Ca_SR * iq), ikc = mrcp(kc), k1 = T(0.15) * ikc;
+        const T w = k1 * Ca_ss * Ca_ss, iw = mrcp(k3 + w), O = w * Rp * iw, grad = Ca_SR - Ca_ss;
         const T Irel = V_rel * O * grad;
-        const T IbCa = T(0.000592) * (V - T(0.5f) * RTF * mlog(Cao / Ca_i)), IpCa = T(0.1238) * Ca_i / kp;
-        const T nao3 = Nao * Nao * Nao, em = mexp((T(0.35) - T(1)) * V * FRT);
-        const T INaCa = T(1000) * (mexp(T(0.35) * V * FRT) * (Na_i * Na_i * Na_i) * Cao - em * nao3 * Ca_i * T(2.5)) /
-                        ((T(87.5) * T(87.5) * T(87.5) + nao3) * (T(1.38) + Cao) * (T(1) + T(0.1) * em));
-        const T sc_ = ((i_leak - i_up) * V_sr) / V_c + i_xfer - ((IbCa + IpCa - T(2) * INaCa) * Cm) / (T(2) * V_c * F);
+        const T IbCa = T(0.000592) * (V - T(0.5f) * RTF * mlog(mdiv(Cao, Ca_i))), IpCa = T(0.1238) * Ca_i * kp;
+        const T sc_ = (i_leak - i_up) * (V_sr / V_c) + i_xfer - (IbCa + IpCa - T(2) * INaCa) * (Cm / (T(2) * V_c * F));
         const T ssr = i_up - (Irel + i_leak);
-        const T sss = (-gd * G * Cm) / (T(2) * V_ss * F) + (Irel * V_sr) / V_ss - (i_xfer * V_c) / V_ss;
-        bcai += aCai * (double)(sc_ * Bc * Bc * T(2) * qc / (cbc * cbc * cbc));
-        bsr += aSR * (double)(ssr * Bsr * Bsr * T(2) * qsr / (cbs * cbs * cbs));
-        bss += aSS * (double)(sss * Bss * Bss * T(2) * qss / (cbss * cbss * cbss));
+        const T sss = -gd * G * (Cm / (T(2) * V_ss * F)) + Irel * (V_sr / V_ss) - i_xfer * (V_c / V_ss);
+        bcai += aCai * (double)(sc_ * T(2) * qc * cbc * ic * ic);
+        bsr += aSR * (double)(ssr * T(2) * qsr * cbs * isr * isr);
+        bss += aSS * (double)(sss * T(2) * qss * cbss * iss * iss);
         // fluxes
         const double uc = aCai * (double)Bc, us = aSR * (double)Bsr, uss = aSS * (double)Bss;
         const double vr = (double)(V_sr / V_c);
         const double bup = us - uc * vr, bleak = uc * vr - us, bx = uc - uss * (double)(V_c / V_ss);
         const double brel = uss * (double)(V_sr / V_ss) - us;
-        bcai += bup * (double)(T(0.006375) * up * up * T(2) * K_up2 / (Ca_i * Ca_i * Ca_i));
+        bcai += bup * (double)(T(0.006375) * T(2) * K_up2 * Ca_i * iu * iu);
         bsr += bleak * (double)T(0.00036f);
         bcai -= bleak * (double)T(0.00036f);
         bss += bx * (double)T(0.0038f);
@@ -227,22 +230,21 @@ __device__ __forceinline__ void adj_cell(const T (&y)[TT_NEQ], const TTScale<T> 
         const T k2 = T(0.045f) * kc;
         brp += bO * (double)(w * iw) - aRp * (double)(k2 * Ca_ss + k4);
         bss += bw * (double)(T(2) * k1 * Ca_ss) - aRp * (double)(k2 * Rp);
-        const double bkc = -aRp * (double)(T(0.045f) * Ca_ss * Rp) - bw * (double)(w / kc);
-        bsr -= bkc * (double)(T(1.5) * T(2) * q2 * iq * iq / Ca_SR);
+        const double bkc = -aRp * (double)(T(0.045f) * Ca_ss * Rp) - bw * (double)(w * ikc);
+        bsr -= bkc * (double)(T(1.5) * T(2) * T(1.5) * T(1.5) * Ca_SR * iq * iq);
     }
-    // gates: inf + (y - inf) exp(-dt / tau)
+    // gates: inf + (y - inf) exp(-dt rate)
     {
-        Dual<T> inf[12], tau[12];
-        tt2006_gate_rates<Dual<T>>(Dual<T>(V, T(1)), Dual<T>(Ca_ss, T(0)), inf, tau);
-        // fCass follows Ca_ss: inf = 0.6 / (1 + c^2) + 0.4, tau = 80 / (1 + c^2) + 2, c = Ca_ss / 0.05
-        const T c = Ca_ss / T(0.05f), ic = T(1) / (T(1) + c * c), dc = -T(2) * c / T(0.05f) * ic * ic;
+        Dual<T> inf[12], rate[12];
+        tt2006_gate_rates<Dual<T>>(Dual<T>(V, T(1)), Dual<T>(Ca_ss, T(0)), inf, rate);
+        // fCass follows Ca_ss: inf = 0.6 / (1 + c^2) + 0.4, 1/rate = 80 / (1 + c^2) + 2, c = Ca_ss / 0.05
+        const T c = MB_OVER(Ca_ss, (double)0.05f), fc = mrcp(T(1) + c * c), dc = -T(2) * MB_OVER(c, (double)0.05f) * fc * fc;
         inf[9].d = T(0.6f) * dc;
-        tau[9].d = T(80.0f) * dc;
+        rate[9].d = -T(80.0f) * dc * rate[9].v * rate[9].v;
 #pragma unroll
         for (int k = 0; k < 12; ++k) {
-            const T E = mexp(-dt / tau[k].v);
-            const double b = g[1 + k] * (double)((T(1) - E) * inf[k].d + (y[1 + k] - inf[k].v) * E *
-                                                 (dt * tau[k].d / (tau[k].v * tau[k].v)));
+            const T E = mexp(-dt * rate[k].v);
+            const double b = g[1 + k] * (double)((T(1) - E) * inf[k].d - (y[1 + k] - inf[k].v) * E * (dt * rate[k].d));
             if (k == 9) bss += b;
             else bV += b;
             res[1 + k] += g[1 + k] * (double)E;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tt2006(mb_ode_dev o, const 
                                                             const double *__restrict__ w, double alpha,
                                                             const double *__restrict__ mu_in, double *mu_out,
                                                             double *lam_out, double *gth) {
+    exp_table_fill();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= o.n) return;
     const uint32_t g = o.cell ? o.cell[t] : t;

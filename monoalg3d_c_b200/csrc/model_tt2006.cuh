@@ -18,6 +18,9 @@ MB_NS_BEGIN
 
 constexpr int TT_NEQ = 19;
 
+// sqrt(Ko / 5.4f) with Ko = 5.4 a double (the two differ in the 8th digit)
+constexpr double TT_SQRT_KO = 1.0 + 0.5 * (5.4 / (double)5.4f - 1.0);
+
 // Indices of the state rows (the reference sv[] order, _RS_CPU.c:140-158).
 enum TTIdx {
     TT_V = 0, TT_XR1, TT_XR2, TT_XS, TT_M, TT_H, TT_J, TT_D, TT_F, TT_F2, TT_FCASS,
@@ -50,78 +53,66 @@ struct TTUpdate {
     T dCai, dCaSR, dCaSS, dRprime, dNai, dKi;
 };
 
-// Steady states and time constants of gates 1..12 (state order): functions of V,
+// Steady states and rates 1/tau of gates 1..12 (state order): functions of V,
 // for fCass of Ca_ss.
 template <typename T>
-__device__ __forceinline__ void tt2006_gate_rates(const T V, const T Ca_ss, T (&inf)[12], T (&tau)[12]) {
-    // gating variables: steady states and time constants
-    const T xr1_inf = T(1.0f) / (T(1.0f) + mexp((T(-26.0f) - V) / T(7.0f)));
-    const T tau_xr1 = (T(450.0f) / (T(1.0f) + mexp((T(-45.0f) - V) / T(10.0f)))) *
-                      (T(6.0f) / (T(1.0f) + mexp((V + T(30.0f)) / T(11.5f))));
-    const T xr2_inf = T(1.0f) / (T(1.0f) + mexp((V + T(88.0f)) / T(24.0f)));
-    const T tau_xr2 = (T(3.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(20.0f)))) *
-                      (T(1.12f) / (T(1.0f) + mexp((V - T(60.0f)) / T(20.0f))));
-    const T xs_inf = T(1.0f) / (T(1.0f) + mexp((T(-5.0f) - V) / T(14.0f)));
-    const T tau_xs = ((T(1400.0f) / msqrt(T(1.0f) + mexp((T(5.0f) - V) / T(6.0f)))) *
-                      (T(1.0f) / (T(1.0f) + mexp((V - T(35.0f)) / T(15.0f))))) + T(80.0f);
-
-    const T em = T(1.0f) + mexp((T(-56.86f) - V) / T(9.03f));
-    const T m_inf = T(1.0f) / (em * em);
-    const T tau_m = (T(1.0f) / (T(1.0f) + mexp((T(-60.0f) - V) / T(5.0f)))) *
-                    ((T(0.1f) / (T(1.0f) + mexp((V + T(35.0f)) / T(5.0f)))) +
-                     (T(0.1f) / (T(1.0f) + mexp((V - T(50.0f)) / T(200.0f)))));
-
-    const T eh = T(1.0f) + mexp((V + T(71.55f)) / T(7.43f));
-    const T h_inf = T(1.0f) / (eh * eh);
-    const T j_inf = h_inf;
-    T alpha_h, beta_h, alpha_j, beta_j;
-    if (V < T(-40.0f)) {
-        alpha_h = T(0.057f) * mexp((-(V + T(80.0f))) / T(6.8f));
-        beta_h = (T(2.7f) * mexp(T(0.079f) * V)) + (T(310000.0f) * mexp(T(0.3485f) * V));
-        alpha_j = ((((T(-25428.0f)) * mexp(T(0.2444f) * V)) - (T(6.948e-06f) * mexp(T(-0.04391f) * V))) *
-                   (V + T(37.78f))) / (T(1.0f) + mexp(T(0.311f) * (V + T(79.23f))));
-        beta_j = (T(0.02424f) * mexp(T(-0.01052f) * V)) / (T(1.0f) + mexp(T(-0.1378f) * (V + T(40.14f))));
-    } else {
-        alpha_h = T(0.0f);
-        beta_h = T(0.77f) / (T(0.13f) * (T(1.0f) + mexp((V + T(10.66f)) / T(-11.1f))));
-        alpha_j = T(0.0f);
-        beta_j = (T(0.6f) * mexp(T(0.057f) * V)) / (T(1.0f) + mexp(T(-0.1f) * (V + T(32.0f))));
+__device__ __forceinline__ void tt2006_gate_rates(const T V, const T Ca_ss, T (&inf)[12], T (&rate)[12]) {
+    inf[0] = sigm(MB_OVER(T(-26.0f) - V, 7.0f));
+    rate[0] = (T(1.0f) + mexp(MB_OVER(T(-45.0f) - V, 10.0f))) * (T(1.0f) + mexp(MB_OVER(V + T(30.0f), 11.5f))) *
+              T(1.0 / (450.0f * 6.0f));
+    inf[1] = sigm(MB_OVER(V + T(88.0f), 24.0f));
+    rate[1] = (T(1.0f) + mexp(MB_OVER(T(-60.0f) - V, 20.0f))) * (T(1.0f) + mexp(MB_OVER(V - T(60.0f), 20.0f))) *
+              T(1.0 / (3.0 * (double)1.12f));
+    inf[2] = sigm(MB_OVER(T(-5.0f) - V, 14.0f));
+    {
+        // 1400 / (sqrt(e1) e2) + 80
+        const T e = msqrt(T(1.0f) + mexp(MB_OVER(T(5.0f) - V, 6.0f))) * (T(1.0f) + mexp(MB_OVER(V - T(35.0f), 15.0f)));
+        rate[2] = mrcp(T(1400.0f) * mrcp(e) + T(80.0f));
     }
-    const T tau_h = T(1.0f) / (alpha_h + beta_h);
-    const T tau_j = T(1.0f) / (alpha_j + beta_j);
-
-    const T d_inf = T(1.0f) / (T(1.0f) + mexp((T(-8.0f) - V) / T(7.5f)));
-    const T tau_d = ((T(1.4f) / (T(1.0f) + mexp((T(-35.0f) - V) / T(13.0f)))) + T(0.25f)) *
-                        (T(1.4f) / (T(1.0f) + mexp((V + T(5.0f)) / T(5.0f)))) +
-                    (T(1.0f) / (T(1.0f) + mexp((T(50.0f) - V) / T(20.0f))));
-
-    const T e30 = mexp((V + T(30.0f)) / T(10.0f));
+    const T em = sigm(MB_OVER(T(-56.86f) - V, 9.03f));
+    inf[3] = em * em;
+    {
+        // a (0.1 / b + 0.1 / c), a = 1 / e
+        const T b = T(1.0f) + mexp(MB_OVER(V + T(35.0f), 5.0f)), c = T(1.0f) + mexp(MB_OVER(V - T(50.0f), 200.0f));
+        rate[3] = mdiv((T(1.0f) + mexp(MB_OVER(T(-60.0f) - V, 5.0f))) * b * c, T(0.1f) * (b + c));
+    }
+    const T eh = sigm(MB_OVER(V + T(71.55f), 7.43f));
+    inf[4] = eh * eh;
+    inf[5] = inf[4];
+    if (V < T(-40.0f)) {
+        const T alpha_h = T(0.057f) * mexp(MB_OVER(-(V + T(80.0f)), 6.8f));
+        const T beta_h = (T(2.7f) * mexp(T(0.079f) * V)) + (T(310000.0f) * mexp(T(0.3485f) * V));
+        const T alpha_j = mdiv((((T(-25428.0f)) * mexp(T(0.2444f) * V)) - (T(6.948e-06f) * mexp(T(-0.04391f) * V))) *
+                                   (V + T(37.78f)),
+                               T(1.0f) + mexp(T(0.311f) * (V + T(79.23f))));
+        const T beta_j = mdiv(T(0.02424f) * mexp(T(-0.01052f) * V), T(1.0f) + mexp(T(-0.1378f) * (V + T(40.14f))));
+        rate[4] = alpha_h + beta_h;
+        rate[5] = alpha_j + beta_j;
+    } else {
+        rate[4] = mdiv(T(0.77f), T(0.13f) * (T(1.0f) + mexp(MB_OVER(V + T(10.66f), -11.1f))));
+        rate[5] = mdiv(T(0.6f) * mexp(T(0.057f) * V), T(1.0f) + mexp(T(-0.1f) * (V + T(32.0f))));
+    }
+    inf[6] = sigm(MB_OVER(T(-8.0f) - V, 7.5f));
+    rate[6] = mrcp((T(1.4f) * sigm(MB_OVER(T(-35.0f) - V, 13.0f)) + T(0.25f)) * (T(1.4f) * sigm(MB_OVER(V + T(5.0f), 5.0f))) +
+                   sigm(MB_OVER(T(50.0f) - V, 20.0f)));
+    const T e30 = sigm(MB_OVER(V + T(30.0f), 10.0f));
     const T v27 = V + T(27.0f);
-    const T f_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(7.0f)));
-    const T tau_f = (T(1102.5f) * mexp((-(v27 * v27)) / T(225.0f))) +
-                    (T(200.0f) / (T(1.0f) + mexp((T(13.0f) - V) / T(10.0f)))) +
-                    (T(180.0f) / (T(1.0f) + e30)) + T(20.0f);
-    const T f2_inf = (T(0.67f) / (T(1.0f) + mexp((V + T(35.0f)) / T(7.0f)))) + T(0.33f);
-    const T tau_f2 = (T(562.0f) * mexp((-(v27 * v27)) / T(240.0f))) +
-                     (T(31.0f) / (T(1.0f) + mexp((T(25.0f) - V) / T(10.0f)))) +
-                     (T(80.0f) / (T(1.0f) + e30));
-
-    const T cr = Ca_ss / T(0.05f);
-    const T fCass_inf = (T(0.6f) / (T(1.0f) + cr * cr)) + T(0.4f);
-    const T tau_fCass = (T(80.0f) / (T(1.0f) + cr * cr)) + T(2.0f);
-
-    const T s_inf = T(1.0f) / (T(1.0f) + mexp((V + T(20.0f)) / T(5.0f)));
+    inf[7] = sigm(MB_OVER(V + T(20.0f), 7.0f));
+    rate[7] = mrcp((T(1102.5f) * mexp(MB_OVER(-(v27 * v27), 225.0f))) + T(200.0f) * sigm(MB_OVER(T(13.0f) - V, 10.0f)) +
+                   T(180.0f) * e30 + T(20.0f));
+    inf[8] = T(0.67f) * sigm(MB_OVER(V + T(35.0f), 7.0f)) + T(0.33f);
+    rate[8] = mrcp((T(562.0f) * mexp(MB_OVER(-(v27 * v27), 240.0f))) + T(31.0f) * sigm(MB_OVER(T(25.0f) - V, 10.0f)) +
+                   T(80.0f) * e30);
+    const T cr = MB_OVER(Ca_ss, (double)0.05f);
+    const T fc = mrcp(T(1.0f) + cr * cr);
+    inf[9] = T(0.6f) * fc + T(0.4f);
+    rate[9] = mrcp(T(80.0f) * fc + T(2.0f));
+    inf[10] = sigm(MB_OVER(V + T(20.0f), 5.0f));
     const T v45 = V + T(45.0f);
-    const T tau_s = (T(85.0f) * mexp((-(v45 * v45)) / T(320.0f))) +
-                    (T(5.0f) / (T(1.0f) + mexp((V - T(20.0f)) / T(5.0f)))) + T(3.0f);
-    const T r_inf = T(1.0f) / (T(1.0f) + mexp((T(20.0f) - V) / T(6.0f)));
+    rate[10] = mrcp((T(85.0f) * mexp(MB_OVER(-(v45 * v45), 320.0f))) + T(5.0f) * sigm(MB_OVER(V - T(20.0f), 5.0f)) + T(3.0f));
+    inf[11] = sigm(MB_OVER(T(20.0f) - V, 6.0f));
     const T v40 = V + T(40.0f);
-    const T tau_r = (T(9.5f) * mexp((-(v40 * v40)) / T(1800.0f))) + T(0.8f);
-
-    inf[0] = xr1_inf; inf[1] = xr2_inf; inf[2] = xs_inf; inf[3] = m_inf; inf[4] = h_inf; inf[5] = j_inf;
-    inf[6] = d_inf; inf[7] = f_inf; inf[8] = f2_inf; inf[9] = fCass_inf; inf[10] = s_inf; inf[11] = r_inf;
-    tau[0] = tau_xr1; tau[1] = tau_xr2; tau[2] = tau_xs; tau[3] = tau_m; tau[4] = tau_h; tau[5] = tau_j;
-    tau[6] = tau_d; tau[7] = tau_f; tau[8] = tau_f2; tau[9] = tau_fCass; tau[10] = tau_s; tau[11] = tau_r;
+    rate[11] = mrcp((T(9.5f) * mexp(MB_OVER(-(v40 * v40), 1800.0f))) + T(0.8f));
 }
 
 // y: the 19 state values (in T), stim: merged stimulus current.
@@ -140,7 +131,7 @@ __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTSca
     const T R = T(8314.472), Tk = T(310.0), F = T(96485.3415f);
     const T Cm = T(0.185), V_c = T(0.016404);
     const T Ko = T(5.4), Nao = T(140.0), Cao = T(2.0);
-    const T P_kna = T(0.03), K_mk = T(1.0), P_NaK = T(2.724), K_mNa = T(40.0), K_pCa = T(0.0005);
+    const T P_kna = T(0.03), K_mNa = T(40.0), K_pCa = T(0.0005);
     // calcium handling
     const T V_rel = T(0.102), k1_prime = T(0.15), max_sr = T(2.5), min_sr = T(1.0);
     const T EC = T(1.5), Vmax_up = T(0.006375);
@@ -153,23 +144,23 @@ __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTSca
     const T g_bca = T(0.000592), g_pCa = T(0.1238), g_K1 = T(5.405) * sc.gK1, g_bna = T(0.00029);
 
     const T RTF = (R * Tk) / F;
-    const T EK = RTF * mlog(Ko / K_i);
-    const T EKs = RTF * mlog((Ko + (P_kna * Nao)) / (K_i + (P_kna * Na_i)));
-    const T ENa = RTF * mlog(Nao / Na_i);
-    const T ECa = ((T(0.5f) * R * Tk) / F) * mlog(Cao / Ca_i);
+    const T EK = RTF * mlog(mdiv(Ko, K_i));
+    const T EKs = RTF * mlog(mdiv(Ko + (P_kna * Nao), K_i + (P_kna * Na_i)));
+    const T ENa = RTF * mlog(mdiv(Nao, Na_i));
+    const T ECa = ((T(0.5f) * R * Tk) / F) * mlog(mdiv(Cao, Ca_i));
 
     // inward rectifier
     const T vek = V - EK;
-    const T beta_K1 = ((T(3.0f) * mexp(T(0.0002f) * (vek + T(100.0f)))) + mexp(T(0.1f) * (vek - T(10.0f)))) /
-                      (T(1.0f) + mexp(T(-0.5f) * vek));
-    const T alpha_K1 = T(0.1f) / (T(1.0f) + mexp(T(0.06f) * (vek - T(200.0f))));
-    const T xK1_inf = alpha_K1 / (alpha_K1 + beta_K1);
+    const T beta_K1 = mdiv((T(3.0f) * mexp(T(0.0002f) * (vek + T(100.0f)))) + mexp(T(0.1f) * (vek - T(10.0f))),
+                           T(1.0f) + mexp(T(-0.5f) * vek));
+    const T alpha_K1 = T(0.1f) * sigm(T(0.06f) * (vek - T(200.0f)));
+    const T xK1_inf = mdiv(alpha_K1, alpha_K1 + beta_K1);
 
     const T IK1 = g_K1 * xK1_inf * vek;
     const T Ito = g_to * r * s * vek;
-    const T IKr = g_Kr * Xr1 * Xr2 * vek * msqrt(Ko / T(5.4f));
+    const T IKr = g_Kr * Xr1 * Xr2 * vek * T(TT_SQRT_KO);
     const T IKs = g_Ks * (Xs * Xs) * (V - EKs);
-    const T IpK = (g_pK * vek) / (T(1.0f) + mexp((T(25.0f) - V) / T(5.98f)));
+    const T IpK = (g_pK * vek) * sigm(MB_OVER(T(25.0f) - V, (double)5.98f));
 
     // L-type calcium current; the removable singularity at V = 15 mV uses
     // the limit value inside a +-1e-5 mV band (_RS_CPU.c:221)
@@ -177,68 +168,69 @@ __device__ __forceinline__ void tt2006_rhs(const T *y, T stim, T dt, const TTSca
     T ICaL;
     const T v15 = V - T(15.0f);
     if (V < T(15.0f - 1.0e-5f) || V > T(15.0f + 1.0e-5f)) {
-        const T ea = (T(2.0f) * v15 * F) / (R * Tk);
-        ICaL = (((g_CaL * d * f * f2 * fCass * T(4.0f) * v15 * (F * F)) / (R * Tk)) *
-                ((T(0.25f) * Ca_ss * mexp(ea)) - Cao)) / mexpm1(ea);
+        const T ea = T(2.0f) * v15 * FRT;
+        ICaL = mdiv((g_CaL * d * f * f2 * fCass * T(4.0f) * v15 * F * FRT) * ((T(0.25f) * Ca_ss * mexp(ea)) - Cao),
+                    mexpm1(ea));
     } else {
         ICaL = g_CaL * d * f * f2 * fCass * T(2.0f) * F * (T(0.25f) * Ca_ss - Cao);
     }
     const T IbCa = g_bca * (V - ECa);
-    const T IpCa = (g_pCa * Ca_i) / (Ca_i + K_pCa);
+    const T IpCa = mdiv(g_pCa * Ca_i, Ca_i + K_pCa);
 
-    const T INaK = ((((P_NaK * Ko) / (Ko + K_mk)) * Na_i) / (Na_i + K_mNa)) /
-                   (T(1.0f) + (T(0.1245f) * mexp(((T(-0.1f)) * V * F) / (R * Tk))) +
-                    (T(0.0353f) * mexp(((-V) * F) / (R * Tk))));
+    // P_NaK Ko / (Ko + K_mk) = 2.724 x 5.4 / 6.4
+    const T INaK = mdiv(T(2.724 * 5.4 / (5.4 + 1.0)) * Na_i,
+                        (Na_i + K_mNa) * (T(1.0f) + (T(0.1245f) * mexp(T(-0.1f) * V * FRT)) +
+                                          (T(0.0353f) * mexp(-V * FRT))));
     const T INa = g_Na * (m * m * m) * h * j * (V - ENa);
     const T IbNa = g_bna * (V - ENa);
-    const T e_gm1 = mexp(((n_gamma - T(1.0f)) * V * F) / (R * Tk));
-    const T INaCa = (K_NaCa * ((mexp((n_gamma * V * F) / (R * Tk)) * (Na_i * Na_i * Na_i) * Cao) -
-                               (e_gm1 * (Nao * Nao * Nao) * Ca_i * n_alpha))) /
-                    (((Km_Nai * Km_Nai * Km_Nai) + (Nao * Nao * Nao)) * (Km_Ca + Cao) *
-                     (T(1.0f) + (K_sat * e_gm1)));
-    (void)FRT;
+    const T e_gm1 = mexp((n_gamma - T(1.0f)) * V * FRT);
+    const T INaCa = mdiv(K_NaCa * ((mexp(n_gamma * V * FRT) * (Na_i * Na_i * Na_i) * Cao) -
+                                   (e_gm1 * (Nao * Nao * Nao) * Ca_i * n_alpha)),
+                         ((Km_Nai * Km_Nai * Km_Nai) + (Nao * Nao * Nao)) * (Km_Ca + Cao) *
+                             (T(1.0f) + (K_sat * e_gm1)));
 
-    T inf[12], tau[12];
-    tt2006_gate_rates<T>(V, Ca_ss, inf, tau);
+    T inf[12], rate[12];
+    tt2006_gate_rates<T>(V, Ca_ss, inf, rate);
 
     // calcium dynamics
-    const T ecs = EC / Ca_SR;
-    const T kcasr = max_sr - ((max_sr - min_sr) / (T(1.0f) + ecs * ecs));
-    const T k1 = k1_prime / kcasr;
+    // x / (x + c) in place of 1 / (1 + c / x)
+    const T sr2 = Ca_SR * Ca_SR;
+    const T kcasr = max_sr - (max_sr - min_sr) * mdiv(sr2, sr2 + EC * EC);
+    const T k1 = mdiv(k1_prime, kcasr);
     const T k3 = T(0.06);
     const T css2 = Ca_ss * Ca_ss;
-    const T O = (k1 * css2 * R_prime) / (k3 + (k1 * css2));
+    const T O = mdiv(k1 * css2 * R_prime, k3 + (k1 * css2));
     const T Irel = V_rel * O * (Ca_SR - Ca_ss);
     const T K_up = T(0.00025);
-    const T i_up = Vmax_up / (T(1.0f) + ((K_up * K_up) / (Ca_i * Ca_i)));
+    const T ci2 = Ca_i * Ca_i;
+    const T i_up = Vmax_up * mdiv(ci2, ci2 + K_up * K_up);
     const T i_leak = T(0.00036f) * (Ca_SR - Ca_i);
     const T i_xfer = T(0.0038f) * (Ca_ss - Ca_i);
     const T k2 = T(0.045f) * kcasr;
     const T k4 = T(0.005f);
     const T Buf_c = T(0.2f), K_buf_c = T(0.001f);
     const T cbc = Ca_i + K_buf_c;
-    const T Ca_i_bufc = T(1.0f) / (T(1.0f) + ((Buf_c * K_buf_c) / (cbc * cbc)));
+    const T Ca_i_bufc = mdiv(cbc * cbc, cbc * cbc + Buf_c * K_buf_c);
     const T K_buf_sr = T(0.3f), Buf_sr = T(10.0f);
     const T cbs = Ca_SR + K_buf_sr;
-    const T Ca_sr_bufsr = T(1.0f) / (T(1.0f) + ((Buf_sr * K_buf_sr) / (cbs * cbs)));
+    const T Ca_sr_bufsr = mdiv(cbs * cbs, cbs * cbs + Buf_sr * K_buf_sr);
     const T Buf_ss = T(0.4f), K_buf_ss = T(0.00025f);
     const T cbss = Ca_ss + K_buf_ss;
-    const T Ca_ss_bufss = T(1.0f) / (T(1.0f) + ((Buf_ss * K_buf_ss) / (cbss * cbss)));
+    const T Ca_ss_bufss = mdiv(cbss * cbss, cbss * cbss + Buf_ss * K_buf_ss);
     const T V_sr = T(0.001094f), V_ss = T(5.468e-05f);
 
     u.dV = -(IK1 + Ito + IKr + IKs + ICaL + INaK + INa + IbNa + INaCa + IbCa + IpK + IpCa + stim);
     u.dRprime = ((-k2) * Ca_ss * R_prime) + (k4 * (T(1.0f) - R_prime));
-    u.dCai = Ca_i_bufc * (((((i_leak - i_up) * V_sr) / V_c) + i_xfer) -
-                          ((((IbCa + IpCa) - (T(2.0f) * INaCa)) * Cm) / (T(2.0f) * V_c * F)));
+    u.dCai = Ca_i_bufc * (((i_leak - i_up) * (V_sr / V_c) + i_xfer) -
+                          ((IbCa + IpCa) - (T(2.0f) * INaCa)) * (Cm / (T(2.0f) * V_c * F)));
     u.dCaSR = Ca_sr_bufsr * (i_up - (Irel + i_leak));
-    u.dCaSS = Ca_ss_bufss * (((((-ICaL) * Cm) / (T(2.0f) * V_ss * F)) + ((Irel * V_sr) / V_ss)) -
-                             ((i_xfer * V_c) / V_ss));
-    u.dNai = ((-(INa + IbNa + (T(3.0f) * INaK) + (T(3.0f) * INaCa))) / (V_c * F)) * Cm;
-    u.dKi = ((-((IK1 + Ito + IKr + IKs + IpK + stim) - (T(2.0f) * INaK))) / (V_c * F)) * Cm;
+    u.dCaSS = Ca_ss_bufss * (((-ICaL) * (Cm / (T(2.0f) * V_ss * F)) + Irel * (V_sr / V_ss)) - i_xfer * (V_c / V_ss));
+    u.dNai = -(INa + IbNa + (T(3.0f) * INaK) + (T(3.0f) * INaCa)) * (Cm / (V_c * F));
+    u.dKi = -((IK1 + Ito + IKr + IKs + IpK + stim) - (T(2.0f) * INaK)) * (Cm / (V_c * F));
 
     // Rush-Larsen gate updates
 #pragma unroll
-    for (int k = 0; k < 12; ++k) u.gate[k] = inf[k] + (y[TT_XR1 + k] - inf[k]) * mexp(-dt / tau[k]);
+    for (int k = 0; k < 12; ++k) u.gate[k] = inf[k] + (y[TT_XR1 + k] - inf[k]) * mexp(-dt * rate[k]);
 }
 
 MB_NS_END

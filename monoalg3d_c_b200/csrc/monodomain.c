@@ -139,6 +139,7 @@ int mb_ode_create(mb_ode **out, int model, int precision, int rl_rule, uint32_t 
     o->dev.n = num_cells;
     o->dev.ld = round_up32(num_cells);
     o->dev.dt = dt;
+    o->dev.variant = mbk_ode_default_variant(model, o->dev.precision, num_cells, (int)num_steps);
     int n64, n32;
     ode_rows(model, precision, 0, &n64, &n32);
     cudaError_t e = cudaStreamCreateWithFlags(&o->stream, cudaStreamNonBlocking);
@@ -268,6 +269,7 @@ int mb_ode_set_steps(mb_ode *o, double dt, uint32_t num_steps) {
     if (!o || !(dt > 0.0) || num_steps == 0) return set_err(MB_ERR_ARG, "bad arguments");
     o->dev.dt = dt;
     o->dev.num_steps = (int)num_steps;
+    o->dev.variant = mbk_ode_default_variant(o->dev.model, o->dev.precision, o->dev.n, (int)num_steps);
     return MB_OK;
 }
 

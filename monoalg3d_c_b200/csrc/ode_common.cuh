@@ -126,6 +126,7 @@ template <int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
 k_tt2006_fp64(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
               double *__restrict__ vout) {
+    exp_table_fill();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= o.n) return;
     const uint32_t g = o.cell ? o.cell[t] : t;
@@ -214,63 +215,166 @@ k_tt2006_mixed(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__r
 // FP64 layout: sv64 row s = state s.
 // Mixed layout: sv64 rows {V, cass, nai, nass, ki, kss, cansr, cajsr, cai},
 //               sv32 rows {CaMKt, states 10..42}.
+
+// Where torord_step finds a cell's state: in rows of in / in32 (element
+// stride ild between rows, the pointers at the cell's column) and where it
+// leaves it, rows of out / out32 and *vout.  The stores may alias later loads as
+// far as the compiler knows, so a part's reads stay behind the stores of the
+// part before it, as the register budget wants.
+struct TorRows64 {
+    const double *in;
+    double *out, *vout;
+    size_t ild, wld;
+    double v, dt;
+    __device__ __forceinline__ double get(int s) const { return s == 0 ? v : in[s * ild]; }
+    __device__ __forceinline__ void put(int s, double y) { out[s * wld] = y; }
+    __device__ __forceinline__ void euler(int s, double y, double d) {
+        if (s == 0) *vout = dt * d + y;
+        else out[s * wld] = dt * d + y;
+    }
+    __device__ __forceinline__ void fence() const { asm volatile("" ::: "memory"); }
+};
+
+struct TorRowsMixed {
+    const double *in;
+    const float *in32;
+    double *out, *vout;
+    float *out32;
+    size_t ild, wld;
+    double v, dt;
+    __device__ __forceinline__ float get(int s) const {
+        bool is64 = false;
+        const int row = tor_mixed_row(s, is64);
+        return s == 0 ? (float)v : (is64 ? (float)in[row * ild] : in32[row * ild]);
+    }
+    __device__ __forceinline__ void put(int s, float y) {
+        bool is64 = false;
+        out32[tor_mixed_row(s, is64) * wld] = y;
+    }
+    // the FP64 rows are read again: the step used them rounded to float
+    __device__ __forceinline__ void euler(int s, float y, float d) {
+        bool is64 = false;
+        const int row = tor_mixed_row(s, is64);
+        if (s == 0) *vout = dt * (double)d + v;
+        else if (is64) out[row * wld] = dt * (double)d + in[row * ild];
+        else out32[row * wld] = (float)dt * d + y;
+    }
+    __device__ __forceinline__ void fence() const { asm volatile("" ::: "memory"); }
+};
+
+// The state in registers, for several sub-steps per call.
+struct TorRegs64 {
+    double y[TOR_NEQ];
+    double dt;
+    __device__ __forceinline__ double get(int s) const { return y[s]; }
+    __device__ __forceinline__ void put(int s, double x) { y[s] = x; }
+    __device__ __forceinline__ void euler(int s, double x, double d) { y[s] = dt * d + x; }
+    __device__ __forceinline__ void fence() const {}
+};
+
+struct TorRegsMixed {
+    double d[TOR_N64];
+    float f[TOR_N32];
+    double dt;
+    __device__ __forceinline__ float get(int s) const {
+        bool is64 = false;
+        const int row = tor_mixed_row(s, is64);
+        return is64 ? (float)d[row] : f[row];
+    }
+    __device__ __forceinline__ void put(int s, float y) {
+        bool is64 = false;
+        f[tor_mixed_row(s, is64)] = y;
+    }
+    __device__ __forceinline__ void euler(int s, float y, float g) {
+        bool is64 = false;
+        const int row = tor_mixed_row(s, is64);
+        if (is64) d[row] = dt * (double)g + d[row];
+        else f[row] = (float)dt * g + y;
+    }
+    __device__ __forceinline__ void fence() const {}
+};
+
+// FP64, one sub-step per call: the rows stream through the step.  Bound by the
+// FP64 pipe and the latency of its chains: 461 us for 2 M cells, the pipe 49 % busy
+// with 2106 FP64 instructions per cell (2237 us and 18 % with 3910 when the 43
+// states and 26 coefficient pairs were held in registers and exp and the
+// divisions were the CUDA library's).
 template <int RULE, int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
-k_torord_fp64(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
-              double *__restrict__ vout) {
+k_torord_fp64(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
+    exp_table_fill();
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= o.n) return;
+    const uint32_t g = o.cell ? o.cell[t] : t;
+    const double stim = cell_stim(o, ctrl, t);
+    const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
+    TorRows64 io{o.sv64 + t, out64(o) + t, vout + g, o.ld, out_ld(o), src[g], o.dt};
+    act_track(o, ctrl, t, io.v);
+    TorScale<double> sc;
+    load_tor_scale(o.scale, o.ld, t, sc);
+    torord_step<double, RULE>(io, stim, o.dt, o.celltype ? (int)o.celltype[t] : 0, sc);
+}
+
+// FP64, several sub-steps per call: the state stays in registers between them.
+template <int RULE, int MINB>
+__global__ void __launch_bounds__(ODE_THREADS, MINB)
+k_torord_fp64_multi(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
+    exp_table_fill();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= o.n) return;
     const uint32_t g = o.cell ? o.cell[t] : t;
     const double stim = cell_stim(o, ctrl, t);
     const size_t ld = o.ld;
     const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
-    double y[TOR_NEQ];
-    y[0] = src[g];
-    act_track(o, ctrl, t, y[0]);
+    TorRegs64 io;
+    io.dt = o.dt;
+    io.y[0] = src[g];
+    act_track(o, ctrl, t, io.y[0]);
 #pragma unroll
-    for (int s = 1; s < TOR_NEQ; ++s) y[s] = o.sv64[s * ld + t];
-    const double celltype = o.celltype ? (double)o.celltype[t] : 0.0;
+    for (int s = 1; s < TOR_NEQ; ++s) io.y[s] = o.sv64[s * ld + t];
+    const int celltype = o.celltype ? (int)o.celltype[t] : 0;
     TorScale<double> sc;
     load_tor_scale(o.scale, ld, t, sc);
-    const double dt = o.dt;
-    for (int step = 0; step < o.num_steps; ++step) torord_rl_step<double, double, RULE>(y, stim, dt, celltype, sc);
-    vout[g] = y[0];
+    for (int step = 0; step < o.num_steps; ++step) torord_step<double, RULE>(io, stim, o.dt, celltype, sc);
+    vout[g] = io.y[0];
     double *w = out64(o);
     const size_t wl = out_ld(o);
 #pragma unroll
-    for (int s = 1; s < TOR_NEQ; ++s) w[s * wl + t] = y[s];
+    for (int s = 1; s < TOR_NEQ; ++s) w[s * wl + t] = io.y[s];
 }
 
+// Mixed: the state of 43 values fits in 76 registers, all its loads are in
+// flight together.
 template <int RULE, int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
-k_torord_mixed(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
-               double *__restrict__ vout) {
+k_torord_mixed(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= o.n) return;
     const uint32_t g = o.cell ? o.cell[t] : t;
     const double stim = cell_stim(o, ctrl, t);
     const size_t ld = o.ld;
     const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
-    TorMixedState st;
-    st.d[0] = src[g];
-    act_track(o, ctrl, t, st.d[0]);
+    TorRegsMixed io;
+    io.dt = o.dt;
+    io.d[0] = src[g];
+    act_track(o, ctrl, t, io.d[0]);
 #pragma unroll
-    for (int r = 1; r < TOR_N64; ++r) st.d[r] = o.sv64[r * ld + t];
+    for (int r = 1; r < TOR_N64; ++r) io.d[r] = o.sv64[r * ld + t];
 #pragma unroll
-    for (int r = 0; r < TOR_N32; ++r) st.f[r] = o.sv32[r * ld + t];
-    const float celltype = o.celltype ? (float)o.celltype[t] : 0.0f;
+    for (int r = 0; r < TOR_N32; ++r) io.f[r] = o.sv32[r * ld + t];
+    const int celltype = o.celltype ? (int)o.celltype[t] : 0;
     TorScale<float> sc;
     load_tor_scale(o.scale, ld, t, sc);
-    const double dt = o.dt;
-    for (int step = 0; step < o.num_steps; ++step) torord_mixed_step<RULE>(st, stim, dt, celltype, sc);
-    vout[g] = st.d[0];
+    for (int step = 0; step < o.num_steps; ++step)
+        torord_step<float, RULE>(io, (float)stim, (float)o.dt, celltype, sc);
+    vout[g] = io.d[0];
     double *w = out64(o);
     float *w32 = out32(o);
     const size_t wl = out_ld(o);
 #pragma unroll
-    for (int r = 1; r < TOR_N64; ++r) w[r * wl + t] = st.d[r];
+    for (int r = 1; r < TOR_N64; ++r) w[r * wl + t] = io.d[r];
 #pragma unroll
-    for (int r = 0; r < TOR_N32; ++r) w32[r * wl + t] = st.f[r];
+    for (int r = 0; r < TOR_N32; ++r) w32[r * wl + t] = io.f[r];
 }
 
 // ---- staged persistent form ----------------------------------------------
@@ -341,9 +445,10 @@ __device__ __forceinline__ double stim_ahead(const mb_ode_dev &o, const mb_ctrl 
 }
 
 // The persistent tile loop: work(t, ahead, d, f) integrates cell t from its
-// state d (N64 doubles, d[0] = V) and f (N32 floats) and stores the results.
+// slots d (N64 doubles, ODE_THREADS apart, the first V) and f (N32 floats) and
+// stores the results.
 template <int N64, int N32, typename W>
-__device__ __forceinline__ void staged_cells(const mb_ode_dev &o, const double *__restrict__ src, W work) {
+__device__ __forceinline__ void staged_slots(const mb_ode_dev &o, const double *__restrict__ src, W work) {
     extern __shared__ __align__(16) unsigned char ode_smem[];
     double *b64 = reinterpret_cast<double *>(ode_smem);
     float *b32 = reinterpret_cast<float *>(ode_smem + (size_t)2 * N64 * ODE_THREADS * 8);
@@ -373,13 +478,7 @@ __device__ __forceinline__ void staged_cells(const mb_ode_dev &o, const double *
         cpa_wait1();
         const uint32_t t = tile * T + tid;
         if (t < o.n) {
-            double d[N64];
-            float f[N32 > 0 ? N32 : 1];
-#pragma unroll
-            for (int r = 0; r < N64; ++r) d[r] = b64[(size_t)(b * N64 + r) * T + tid];
-#pragma unroll
-            for (int r = 0; r < N32; ++r) f[r] = b32[(size_t)(b * N32 + r) * T + tid];
-            work(t, cur, d, f);
+            work(t, cur, &b64[(size_t)(b * N64) * T + tid], &b32[(size_t)(b * N32) * T + tid]);
         }
         cur = nxt;
         nxt = after;
@@ -388,10 +487,25 @@ __device__ __forceinline__ void staged_cells(const mb_ode_dev &o, const double *
     cpa_wait0();
 }
 
+// The same with the state handed over in registers.
+template <int N64, int N32, typename W>
+__device__ __forceinline__ void staged_cells(const mb_ode_dev &o, const double *__restrict__ src, W work) {
+    staged_slots<N64, N32>(o, src, [&](uint32_t t, const CellAhead &e, const double *sd, const float *sf) {
+        double d[N64];
+        float f[N32 > 0 ? N32 : 1];
+#pragma unroll
+        for (int r = 0; r < N64; ++r) d[r] = sd[(size_t)r * ODE_THREADS];
+#pragma unroll
+        for (int r = 0; r < N32; ++r) f[r] = sf[(size_t)r * ODE_THREADS];
+        work(t, e, d, f);
+    });
+}
+
 template <int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
 k_tt2006_fp64_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
                 double *__restrict__ vout) {
+    exp_table_fill();
     const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
     staged_cells<TT_NEQ, 0>(o, src, [&](uint32_t t, const CellAhead &e, double (&y)[TT_NEQ], float (&)[1]) {
         act_track(o, ctrl, t, y[0]);
@@ -470,53 +584,62 @@ k_tt2006_mixed_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *_
 
 template <int RULE, int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
-k_torord_fp64_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
-                double *__restrict__ vout) {
+k_torord_fp64_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
+    exp_table_fill();
     const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
-    staged_cells<TOR_NEQ, 0>(o, src, [&](uint32_t t, const CellAhead &e, double (&y)[TOR_NEQ], float (&)[1]) {
-        act_track(o, ctrl, t, y[0]);
-        const double stim = stim_ahead(o, ctrl, e);
-        const double celltype = (double)(e.bits >> 8);
+    staged_slots<TOR_NEQ, 0>(o, src, [&](uint32_t t, const CellAhead &e, const double *d, const float *) {
+        TorRows64 io{d, out64(o) + t, vout + e.g, ODE_THREADS, out_ld(o), d[0], o.dt};
+        act_track(o, ctrl, t, io.v);
         TorScale<double> sc;
         load_tor_scale(o.scale, o.ld, t, sc);
-        const double dt = o.dt;
-        for (int step = 0; step < o.num_steps; ++step) torord_rl_step<double, double, RULE>(y, stim, dt, celltype, sc);
-        vout[e.g] = y[0];
-        double *w = out64(o);
-        const size_t wl = out_ld(o);
-#pragma unroll
-        for (int s = 1; s < TOR_NEQ; ++s) w[s * wl + t] = y[s];
+        torord_step<double, RULE>(io, stim_ahead(o, ctrl, e), o.dt, (int)(e.bits >> 8), sc);
     });
 }
 
 template <int RULE, int MINB>
 __global__ void __launch_bounds__(ODE_THREADS, MINB)
-k_torord_mixed_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *__restrict__ vin,
-                 double *__restrict__ vout) {
+k_torord_mixed_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
     const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
-    staged_cells<TOR_N64, TOR_N32>(o, src, [&](uint32_t t, const CellAhead &e, double (&d)[TOR_N64],
-                                                float (&f)[TOR_N32]) {
-        TorMixedState st;
-#pragma unroll
-        for (int r = 0; r < TOR_N64; ++r) st.d[r] = d[r];
-#pragma unroll
-        for (int r = 0; r < TOR_N32; ++r) st.f[r] = f[r];
-        act_track(o, ctrl, t, st.d[0]);
-        const double stim = stim_ahead(o, ctrl, e);
-        const float celltype = (float)(e.bits >> 8);
+    staged_slots<TOR_N64, TOR_N32>(o, src, [&](uint32_t t, const CellAhead &e, const double *d, const float *f) {
+        TorRowsMixed io{d, f, out64(o) + t, vout + e.g, out32(o) + t, ODE_THREADS, out_ld(o), d[0], o.dt};
+        act_track(o, ctrl, t, io.v);
         TorScale<float> sc;
         load_tor_scale(o.scale, o.ld, t, sc);
-        const double dt = o.dt;
-        for (int step = 0; step < o.num_steps; ++step) torord_mixed_step<RULE>(st, stim, dt, celltype, sc);
-        vout[e.g] = st.d[0];
-        double *w = out64(o);
-        float *w32 = out32(o);
-        const size_t wl = out_ld(o);
-#pragma unroll
-        for (int r = 1; r < TOR_N64; ++r) w[r * wl + t] = st.d[r];
-#pragma unroll
-        for (int r = 0; r < TOR_N32; ++r) w32[r * wl + t] = st.f[r];
+        torord_step<float, RULE>(io, (float)stim_ahead(o, ctrl, e), (float)o.dt, (int)(e.bits >> 8), sc);
     });
+}
+
+// Mixed, one sub-step per call, one tile per block with the rows copied into
+// shared memory first: every load of a cell is in flight at once, as in the
+// register form, at the register budget of the streaming one (80 registers, no
+// spills, 24 warps per SM).  Bound by HBM: 619 us for 8 M cells (416 B each, 83 % of
+// the measured copy rate) against 658 us for the best register form, 717 us for
+// the best persistent staged one, and 800 us for the register form that held
+// the gates' coefficients as well.
+template <int RULE, int MINB>
+__global__ void __launch_bounds__(ODE_THREADS, MINB)
+k_torord_mixed_slots(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *vin, double *vout) {
+    __shared__ double b64[TOR_N64 * ODE_THREADS];
+    __shared__ float b32[TOR_N32 * ODE_THREADS];
+    const uint32_t tid = threadIdx.x, t = blockIdx.x * ODE_THREADS + tid;
+    if (t >= o.n) return;
+    const uint32_t g = o.cell ? o.cell[t] : t;
+    const size_t ld = o.ld;
+    const double *src = (ctrl == nullptr || ctrl->cur_time > 0.0) ? vin : vout;
+    cpa8(&b64[tid], src + g);
+#pragma unroll
+    for (int r = 1; r < TOR_N64; ++r) cpa8(&b64[r * ODE_THREADS + tid], o.sv64 + r * ld + t);
+#pragma unroll
+    for (int r = 0; r < TOR_N32; ++r) cpa4(&b32[r * ODE_THREADS + tid], o.sv32 + r * ld + t);
+    cpa_commit();
+    const double stim = cell_stim(o, ctrl, t);
+    TorScale<float> sc;
+    load_tor_scale(o.scale, ld, t, sc);
+    const int celltype = o.celltype ? (int)o.celltype[t] : 0;
+    cpa_wait0();
+    TorRowsMixed io{b64 + tid, b32 + tid, out64(o) + t, vout + g, out32(o) + t, ODE_THREADS, out_ld(o), b64[tid], o.dt};
+    act_track(o, ctrl, t, io.v);
+    torord_step<float, RULE>(io, (float)stim, (float)o.dt, celltype, sc);
 }
 
 // Grid of a staged kernel: every SM filled to the occupancy its registers
@@ -535,8 +658,8 @@ inline unsigned staged_grid(const void *fn, size_t smem, unsigned tiles) {
 }
 
 // Launch of one (model, precision) family: variants 0..5 are the one-cell-
-// per-thread kernels with at least 1..6 resident blocks per SM, 6..9 the
-// staged kernels with at least 1..4.  A staged launch that cannot be placed
+// per-thread kernels with at least 1..6 resident blocks per SM (mixed ToRORd:
+// see ode_mixed.cu), 6..9 the staged kernels with at least 1..4.  A staged launch that cannot be placed
 // (shared memory) returns cudaErrorInvalidConfiguration.
 #define MB_VARIANT_SWITCH(variant, LAUNCH, LAUNCH_S) \
     switch (variant) {                               \
@@ -550,6 +673,16 @@ inline unsigned staged_grid(const void *fn, size_t smem, unsigned tiles) {
     case 7: LAUNCH_S(2); break;                      \
     case 8: LAUNCH_S(3); break;                      \
     default: LAUNCH_S(4); break;                     \
+    }
+
+// Launch of the several-sub-steps kernels: the variant only picks the
+// register budget (at least 1 .. 4 resident blocks per SM).
+#define MB_MULTI_SWITCH(variant, LAUNCH) \
+    switch (variant) {                   \
+    case 0: LAUNCH(1); break;            \
+    case 1: LAUNCH(2); break;            \
+    case 2: LAUNCH(3); break;            \
+    default: LAUNCH(4); break;           \
     }
 
 MB_NS_END

@@ -167,6 +167,16 @@ extern "C" int mbk_ode_step(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vi
         MB_VARIANT_SWITCH(o->variant, L, LS)
 #undef L
 #undef LS
+    } else if (o->num_steps > 1) {
+#define L(MB)                                                                                        \
+    do {                                                                                             \
+        if (o->rl_rule == MB_RL_TRUE)                                                                \
+            k_torord_fp64_multi<MB_RL_TRUE, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout);        \
+        else                                                                                         \
+            k_torord_fp64_multi<MB_RL_REFERENCE_CPU, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout); \
+    } while (0)
+        MB_MULTI_SWITCH(o->variant, L)
+#undef L
     } else if (o->rl_rule == MB_RL_TRUE) {
 #define L(MB) k_torord_fp64<MB_RL_TRUE, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout)
 #define LS(MB) MB_STAGED((k_torord_fp64_s<MB_RL_TRUE, MB>), TOR_NEQ, 0)
@@ -182,6 +192,19 @@ extern "C" int mbk_ode_step(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vi
     }
 #undef MB_STAGED
     return (int)cudaGetLastError();
+}
+
+// The variant of an object that is not tuned (mb_ode_create).  Up to two
+// blocks per SM the register budget does not limit what runs at once, so the
+// kernel with the most registers is taken; beyond that FP64 takes 128 registers
+// (200 k ToRORd cells: 56 us, 70 with 196 registers), mixed the highest
+// occupancy that does not spill.
+extern "C" int mbk_ode_default_variant(int model, int precision, uint32_t n, int num_steps) {
+    if (model == MB_MODEL_TORORD_FKATP_ENDO) return 0;
+    if ((n + ODE_THREADS - 1) / ODE_THREADS <= 2 * 148) return 0;
+    if (precision == MB_PREC_FP64) return model != MB_MODEL_TT2006 && num_steps > 1 ? 0 : 3;
+    if (model == MB_MODEL_TT2006) return 5;
+    return num_steps > 1 ? 1 : 4;
 }
 
 extern "C" int mbk_ode_gather(const mb_ode_dev *o, const double *v, double *out_dev, cudaStream_t s) {
@@ -200,4 +223,28 @@ extern "C" double mb_tt2006_default_state(int s) { return tt2006_default_state(s
 extern "C" double mb_torord_default_state(int celltype, int s) { return torord_default_state(celltype, s); }
 extern "C" double mb_torord_endo_default_state(int gpu_build, int s) {
     return gpu_build ? mb_tore::initial_state_gpu(s) : mb_tore::initial_state_cpu(s);
+}
+
+// The cell models' own double functions on host arrays, for their tests:
+// fn 0 mexp(x), 1 mrcp(x), 2 mdiv(x, y).
+__global__ void k_math_eval(int fn, int n, const double *x, const double *y, double *out) {
+    exp_table_fill();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        out[i] = fn == 0 ? mexp(x[i]) : (fn == 1 ? mrcp(x[i]) : mdiv(x[i], y[i]));
+}
+
+extern "C" int mbk_math_eval(int fn, int n, const double *x, const double *y, double *out) {
+    if (n <= 0) return 0;
+    double *d = nullptr;
+    const size_t b = (size_t)n * sizeof(double);
+    cudaError_t e = cudaMalloc((void **)&d, 3 * b);
+    if (e == cudaSuccess) e = cudaMemcpy(d, x, b, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, y, b, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_math_eval<<<148, 128>>>(fn, n, d, d + n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, b, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return (int)e;
 }

@@ -25,16 +25,31 @@ extern "C" int mbk_ode_step_mixed(const mb_ode_dev *o, mb_ctrl *ctrl, const doub
         MB_VARIANT_SWITCH(o->variant, L, LS)
 #undef L
 #undef LS
-    } else if (o->rl_rule == MB_RL_TRUE) {
-#define L(MB) k_torord_mixed<MB_RL_TRUE, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout)
-#define LS(MB) MB_STAGED((k_torord_mixed_s<MB_RL_TRUE, MB>), TOR_N64, TOR_N32)
-        MB_VARIANT_SWITCH(o->variant, L, LS)
-#undef L
-#undef LS
     } else {
-#define L(MB) k_torord_mixed<MB_RL_REFERENCE_CPU, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout)
-#define LS(MB) MB_STAGED((k_torord_mixed_s<MB_RL_REFERENCE_CPU, MB>), TOR_N64, TOR_N32)
-        MB_VARIANT_SWITCH(o->variant, L, LS)
+        // Variants 0 and 1 keep the state in registers (any number of
+        // sub-steps), 2..5 copy it to shared memory first, 6..9 are staged
+        // persistent launches; several sub-steps per call take 0 or 1.
+#define L(R, K, MB) k_torord_mixed##K<R, MB><<<blocks, ODE_THREADS, 0, s>>>(a, ctrl, vin, vout)
+#define LS(R, MB) MB_STAGED((k_torord_mixed_s<R, MB>), TOR_N64, TOR_N32)
+#define ALL(R)                                                        \
+    switch (o->num_steps > 1 && o->variant > 1 ? 1 : o->variant) {    \
+    case 0: L(R, , 1); break;                                         \
+    case 1: L(R, , 4); break;                                         \
+    case 2: L(R, _slots, 4); break;                                   \
+    case 3: L(R, _slots, 5); break;                                   \
+    case 4: L(R, _slots, 6); break;                                   \
+    case 5: L(R, _slots, 7); break;                                   \
+    case 6: LS(R, 1); break;                                          \
+    case 7: LS(R, 2); break;                                          \
+    case 8: LS(R, 3); break;                                          \
+    default: LS(R, 4); break;                                         \
+    }
+        if (o->rl_rule == MB_RL_TRUE) {
+            ALL(MB_RL_TRUE)
+        } else {
+            ALL(MB_RL_REFERENCE_CPU)
+        }
+#undef ALL
 #undef L
 #undef LS
     }
