@@ -199,7 +199,7 @@ typedef struct mb_pcg_dev {
     mb_ctrl *ctrl;
     unsigned *bar;           /* 2 words, zero at start */
     int *status;             /* 0 = ok; set on a barrier timeout */
-    int form;                /* MB_PCG_FLAT, MB_PCG_TILED or MB_PCG_RESIDENT */
+    int form;                /* MB_PCG_* */
     int variant;             /* launch-shape variant of cg_flat.cu */
     int tiles_x, tiles_y, zchunk, nchunks;
     /* resident kernel (cg_resident.cu): shape, tile grid and tile size,
@@ -210,13 +210,19 @@ typedef struct mb_pcg_dev {
     /* z-march kernel (cg_zmarch.cu): variant, per-plane Jacobi tables
      * (nz x 9 row classes) and the device array of its tensor maps */
     int zc_variant;
+    int cc_variant;          /* cluster kernel: 2^cc_variant blocks */
     double *zc_inv64;
     float *zc_inv32;
     float *zc_ptab32;       /* [nz][mbk_zcg_ptab_floats()] per-plane blocks (window Q pass) */
     double *zc_w;           /* A x of the fused solve's last residual (mixed), or NULL */
     void *zc_maps;
 } mb_pcg_dev;
-enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3 };
+enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3, MB_PCG_CLUSTER = 4 };
+int mbk_ccg_variants(void);
+int mbk_ccg_usable(const mb_pcg_dev *p, int variant);
+int mbk_ccg_launch(const mb_pcg_dev *p, cudaStream_t s);
+/* a system for timing the CG kernels: out = vstar + up to 5 mV of noise */
+int mbk_tune_rhs(double *out, const double *vstar, int64_t n, cudaStream_t s);
 int mbk_fcg_variants(int kind);
 int mbk_fcg_variant_groups(int variant);
 int mbk_fcg_max_blocks(int mixed, int kind, int variant);

@@ -434,6 +434,7 @@ static int step_ode(mb_monodomain *m) {
 
 static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
     switch (q->form) {
+    case MB_PCG_CLUSTER: return mbk_ccg_launch(q, s);
     case MB_PCG_TILED: return mbk_tcg_launch(q, s);
     case MB_PCG_RESIDENT: return mbk_rcg_launch(q, s);
     case MB_PCG_ZMARCH: return mbk_zcg_launch(q, s);
@@ -442,13 +443,17 @@ static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
 }
 
 /* Picks the CG kernel: every launch-shape variant of the flat persistent
- * kernel, the 2.5D tiled one, where its tiles fit the resident one and, for
- * the 27-point class-table operator, every variant of the z-march kernel
- * solve the tissue's first system (b = alpha V* from the initial state)
- * twice; V is restored after every trial and the fastest by CUDA events is
- * kept.  MB_CG_VARIANT=<n> forces a choice (n = number of flat variants
- * selects the tiled kernel, n + 1 the resident kernel, n + 2 + v z-march
- * variant v). */
+ * kernel, the 2.5D tiled one, where its tiles fit the resident one, for
+ * the 27-point class-table operator every variant of the z-march kernel and,
+ * where the vectors fit a cluster's shared memory, every cluster size of the
+ * cluster kernel solve one system; V is restored after every trial and the
+ * fastest by CUDA events is kept.  The system is the tissue's first one with up to
+ * 5 mV of noise on V*, so that it takes as many iterations as a step with
+ * wave fronts does (the initial state alone is solved in one or two, which ranks
+ * the kernels by their set-up).  A candidate whose warm-up run takes over 1.5
+ * times the best is not run again.  MB_CG_VARIANT=<n> forces a choice (n = number of
+ * flat variants selects the tiled kernel, n + 1 the resident kernel, n + 2 + v
+ * z-march variant v, and after all of those the cluster of 2^v blocks). */
 static int cg_autotune(mb_monodomain *m) {
     if (!m->use_pcg) return MB_OK;
     const int mixed = m->pcg.mixed;
@@ -466,17 +471,26 @@ static int cg_autotune(mb_monodomain *m) {
     const int zmarch = mbk_zcg_usable(&m->st) && m->pcg.zc_maps != NULL;
     const int nzv = mbk_zcg_variants();
     const char *env = getenv("MB_CG_VARIANT");
-    /* candidates 0..nv-1 flat, nv tiled, nv+1 resident, nv+2.. z-march */
-    int lo = 0, hi = nv + 1 + (zmarch ? nzv : 0);
+    const int ncv = mbk_ccg_variants();
+    /* candidates 0..nv-1 flat, nv tiled, nv+1 resident, nv+2.. z-march, then clusters */
+    int lo = 0, hi = nv + 1 + nzv + ncv;
     if (env) lo = hi = atoi(env);
-    double *vsave = NULL;
+    double *vsave = NULL, *rhs = NULL;
     if (cudaMalloc((void **)&vsave, (size_t)m->n * sizeof(double)) != cudaSuccess)
         return set_err(MB_ERR_NOMEM, "CG tuning buffer");
+    if (cudaMalloc((void **)&rhs, (size_t)m->n * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        rhs = NULL;             /* no room: the initial state's own system */
+    } else if (mbk_tune_rhs(rhs, m->d_vstar, m->n, m->stream)) {
+        cudaFree(vsave); cudaFree(rhs);
+        return set_err(MB_ERR_CUDA, "CG tuning system");
+    }
     cudaMemcpyAsync(vsave, m->d_v, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
     float best = 1e30f;
     int bestc = 0, rc = MB_OK;      /* variant 0 runs on every grid */
     for (int cand = lo; cand <= hi && !rc; ++cand) {
         mb_pcg_dev q = m->pcg;
+        if (rhs) q.vstar = rhs;
         if (cand < nv) {
             q.form = MB_PCG_FLAT;
             q.variant = cand;
@@ -490,8 +504,13 @@ static int cg_autotune(mb_monodomain *m) {
             if (!resident) continue;
             q.form = MB_PCG_RESIDENT;
             q.blocks = q.rc_nbx * q.rc_nby;
+        } else if (cand - nv - 2 >= nzv) {
+            q.form = MB_PCG_CLUSTER;
+            q.cc_variant = cand - nv - 2 - nzv;
+            if (!mbk_ccg_usable(&q, q.cc_variant)) continue;
+            q.blocks = 1 << q.cc_variant;
         } else {
-            if (!zmarch || cand - nv - 2 >= nzv) continue;
+            if (!zmarch) continue;
             q.form = MB_PCG_ZMARCH;
             q.zc_variant = cand - nv - 2;
             q.blocks = mbk_zcg_max_blocks(mixed, q.zc_variant);
@@ -513,6 +532,7 @@ static int cg_autotune(mb_monodomain *m) {
             float ms = 0;
             cudaEventElapsedTime(&ms, m->ev[0], m->ev[1]);
             if (rep > 0) tsum += ms;      /* first run warms up */
+            else if (ms > 0.75f * best) { tsum = 1e30f; break; }
         }
         if (!rc && tsum < best) {
             best = tsum;
@@ -523,6 +543,7 @@ static int cg_autotune(mb_monodomain *m) {
     forget_stored_product(m);
     cudaStreamSynchronize(m->stream);
     cudaFree(vsave);
+    cudaFree(rhs);
     if (rc) return rc;
     int st = 0;
     cudaMemcpy(&st, m->d_status, sizeof st, cudaMemcpyDeviceToHost);
@@ -539,6 +560,10 @@ static int cg_autotune(mb_monodomain *m) {
     } else if (bestc == nv + 1) {
         m->pcg.form = MB_PCG_RESIDENT;
         m->pcg.blocks = m->pcg.rc_nbx * m->pcg.rc_nby;
+    } else if (bestc - nv - 2 >= nzv) {
+        m->pcg.form = MB_PCG_CLUSTER;
+        m->pcg.cc_variant = bestc - nv - 2 - nzv;
+        m->pcg.blocks = 1 << m->pcg.cc_variant;
     } else {
         m->pcg.form = MB_PCG_ZMARCH;
         m->pcg.zc_variant = bestc - nv - 2;
@@ -1081,7 +1106,8 @@ int mb_monodomain_tuning(mb_monodomain *m, int *ode_variant, int *cg_blocks, int
         *cg_kernel = !m->use_pcg ? -1
                    : m->pcg.form == MB_PCG_TILED ? 100
                    : m->pcg.form == MB_PCG_RESIDENT ? 200
-                   : m->pcg.form == MB_PCG_ZMARCH ? 300 + m->pcg.zc_variant : m->pcg.variant;
+                   : m->pcg.form == MB_PCG_ZMARCH ? 300 + m->pcg.zc_variant
+                   : m->pcg.form == MB_PCG_CLUSTER ? 400 + m->pcg.cc_variant : m->pcg.variant;
     return MB_OK;
 }
 
