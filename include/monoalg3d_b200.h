@@ -430,8 +430,8 @@ int mb_monodomain_time_steps_host_async(mb_monodomain *m, int n, const double *s
  * persistent kernel, 200 = the resident tile-column kernel).  The
  * environment variable MB_CG_VARIANT, read at creation, forces a choice:
  * 0..n-1 a flat shape, n the tiled kernel, n + 1 the resident kernel, n + 2 + v
- * z-march variant v (300 + v), and after those the cluster kernel with 2^v
- * blocks (400 + v). */
+ * z-march variant v (300 + v), then the cluster kernel with 2^v blocks
+ * (400 + v), then the fused flat form's shapes (500 + v). */
 int mb_monodomain_tuning(mb_monodomain *m, int *ode_variant, int *cg_blocks, int *cg_kernel);
 int mb_cg_launch_shapes(int *flat_shapes);
 

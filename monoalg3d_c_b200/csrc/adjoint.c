@@ -217,7 +217,8 @@ int mb_adjoint_backward(mb_adjoint *a, const double *dtraces, double *grad_sigma
             mb_tissue_snapshot_parts(m, snap0, &v0, &sv0, NULL);
             /* A w = lambda_{step+1} (warm start from the previous w) */
             AKK(mbk_adj_tol(a->d_lam, n, 1e-24, a->d_actrl, s));
-            AKK(q.form == MB_PCG_CLUSTER ? mbk_ccg_launch(&q, s) : mbk_fcg_launch(&q, s));
+            AKK(q.form == MB_PCG_CLUSTER ? mbk_ccg_launch(&q, s)
+                : q.form == MB_PCG_FUSED ? mbk_ffcg_launch(&q, s) : mbk_fcg_launch(&q, s));
             /* conductivity gradient through A(sigma) at v_{step+1} */
             AKK(mbk_adj_face_grad(&m->st, a->d_sigma, a->d_w, v1, a->mx, a->my, a->mz, a->d_gsig, s));
             /* through the Rush-Larsen step at (v_step, s_step) */

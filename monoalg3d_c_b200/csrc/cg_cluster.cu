@@ -50,27 +50,7 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, double (&v)[8
                                             double (*wsum)[8], int &red) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned C = cl.num_blocks(), me = cl.block_rank();
-    double a4[4], a2[2], s;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const bool up = (lane & 16u) != 0u;
-        const double keep = up ? v[q + 4] : v[q], give = up ? v[q] : v[q + 4];
-        a4[q] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const bool up = (lane & 8u) != 0u;
-        const double keep = up ? a4[q + 2] : a4[q], give = up ? a4[q] : a4[q + 2];
-        a2[q] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-    }
-    {
-        const bool up = (lane & 4u) != 0u;
-        const double keep = up ? a2[1] : a2[0], give = up ? a2[0] : a2[1];
-        s = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    // lane 4 i holds value ((i & 4) ? 4 : 0) + ((i & 2) ? 2 : 0) + (i & 1) = i
+    const double s = fcg::warp_sum8(v);
     if ((lane & 3u) == 0u) wsum[warp][lane >> 2] = s;
     __syncthreads();
     const int buf = red & 1;

@@ -34,6 +34,7 @@
 // per thread before use, resident blocks per SM); the host times the
 // variants on the tissue's first solve and keeps the fastest.
 #include "cg_rows.cuh"
+#include "mb_math.cuh"
 
 namespace mb {
 namespace fcg {
@@ -590,6 +591,243 @@ __global__ void __launch_bounds__(NT, MINB) k_fcg(Args a) {
     }
 }
 
+// ---- one pass and one reduction per iteration ---------------------------------
+//
+// The fused form keeps z = M r and s = M A p instead of r and A p (M the Jacobi
+// preconditioner), so that the next direction can be formed at every stencil
+// point from three arrays and no diagonal:
+//     z' = z - alpha s,   p' = z' + beta p.
+// A pass forms p' at the row's points, applies A, stores the cell's z', p' and s', applies
+// the last direction's x update (a pass late), and sums, with q = A p' and r = z'/M,
+// p'.q, q.z', q.Mq, q.r, q.q, r.z', r.r; after the reduction alpha = r.z / p.q from
+// the stored z's own sums, and the next r.z and r.r follow as in cg_cluster.cu, with the
+// same guard against cancellation.  z, p and s alternate between two buffers, because
+// other blocks read the ones a pass replaces.
+//
+// Why: while the vectors fit in L2 an iteration of the two-pass form is two
+// grid reductions and two ramps of a pass, more than its memory traffic; the fused
+// form reads as much (three arrays at the row's points against two and a
+// streaming pass) and writes one array less (measured: mbk_ffcg_usable below).
+
+__device__ __forceinline__ double nma(double a, double b, double c) { return fma(-a, b, c); }
+__device__ __forceinline__ float nma(float a, float b, float c) { return fmaf(-a, b, c); }
+__device__ __forceinline__ double ma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float ma(float a, float b, float c) { return fmaf(a, b, c); }
+
+// p' = (z - al s) + bt p, formed where it is read.
+template <typename T>
+struct NextDirection {
+    const T *z, *s, *p;
+    T al, bt;
+    __device__ __forceinline__ Vec4<T> row(uint32_t i) const {
+        const Vec4<T> a = ld4(z, i), b = ld4(s, i), c = ld4(p, i);
+        Vec4<T> o;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o.v[k] = ma(bt, c.v[k], nma(al, b.v[k], a.v[k]));
+        return o;
+    }
+    __device__ __forceinline__ T at(uint32_t i) const { return ma(bt, p[i], nma(al, s[i], z[i])); }
+};
+
+template <bool MIXED, int KIND, int NT, int U, int MINB, bool VEC, int ORD>
+__global__ void __launch_bounds__(NT, MINB) k_ffcg(Args a) {
+    using T = typename Prec<MIXED>::T;
+    constexpr double GUARD = 1e-4;     // as in cg_cluster.cu
+    mb_ctrl *c = a.ctrl;
+    const mb_stencil_dev &st = a.st;
+    const bool pre = c->use_precond != 0;
+    const double tol = c->tol, ratio = c->refine_ratio;
+    const int max_its = c->max_its;
+    // the two buffers of z, p and s
+    auto bz = [&](int i) -> T * { return MIXED ? (T *)(i ? a.r32 : a.z32) : (T *)(i ? a.r64 : a.z64); };
+    auto bp = [&](int i) -> T * { return MIXED ? (T *)(i ? a.pb32 : a.pa32) : (T *)(i ? a.pb64 : a.pa64); };
+    auto bs = [&](int i) -> T * { return MIXED ? (T *)(i ? a.ap32b : a.ap32) : (T *)(i ? a.ap64b : a.ap64); };
+    double *__restrict__ x = a.x;
+    __shared__ T itab[64], dtab[64];
+    if constexpr (KIND == 0) {
+        fill_inv_table<MIXED>(st, itab);
+        __syncthreads();
+        for (unsigned m = threadIdx.x; m < 64; m += blockDim.x) dtab[m] = T(1) / itab[m];
+        __syncthreads();
+    }
+    int red = 0;
+    double v[8];
+    auto zero = [&]() {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    };
+    auto inv = [&](uint32_t g, unsigned m) -> T { return pre ? inv_of<MIXED, KIND>(a, itab, g, m) : T(1); };
+    // r = z / M: with constant coefficients by the code's diagonal
+    auto r_of = [&](T z, T id, unsigned m) -> T {
+        if constexpr (KIND == 0) return pre ? z * dtab[m & 63u] : z;
+        else if constexpr (MIXED) return z / id;
+        else return mdiv(z, id);
+    };
+    // one cell of a pass: zn = z', q = A p'; returns s'
+    auto sums = [&](T pn, T q, T zn, T id, unsigned m) -> T {
+        const T sn = id * q;
+        const double r = (double)r_of(zn, id, m), qd = (double)q, zd = (double)zn;
+        v[0] += (double)pn * qd;
+        v[1] += qd * zd;
+        v[2] += qd * (double)sn;
+        v[3] += qd * r;
+        v[4] += qd * qd;
+        v[5] += r * zd;
+        v[6] += r * r;
+        return sn;
+    };
+    // streaming pass over the active cells: f(g)
+    auto stream = [&](auto f) {
+        const uint32_t n = (uint32_t)st.nx * st.ny * st.nz;
+        const Sweep<ORD> sw(n, blockDim.x);
+        for (uint32_t g = sw.start; g < sw.end; g += sw.step) {
+            const unsigned m = KIND == 2 ? ACTIVE : (unsigned)st.code[g];
+            if (m & ACTIVE) f(g, m);
+        }
+    };
+
+    double t3[3] = {0.0, 0.0, 0.0};
+    residual_pass<MIXED, KIND, NT, U, VEC, ORD>(a, bz(1), bp(0), pre, itab, t3);
+    zero();
+    v[0] = t3[0]; v[1] = t3[1]; v[2] = t3[2];
+    if (!grid_reduce8<NT>(a, v, red)) return;
+    double rz = v[0], rr = v[1], error = v[2], rr_ref = v[2], alpha = 0.0, beta = 0.0;
+    int its = 1, refinements = MIXED ? 1 : 0, pi = 0, zi = 1, si = 1;
+    bool done = !(error >= tol) || !(1 < max_its), first = true, updated = false;
+    const T *zc = bp(0);               // the current z: p itself until the first update
+    while (!done) {
+        const T *po = bp(pi), *so = bs(si);
+        T *zw = bz(zi ^ 1), *pw = bp(pi ^ 1), *sw_ = bs(si ^ 1);
+        const T al = updated ? T(0) : (T)alpha, bt = (T)beta;
+        const double xa = alpha;
+        zero();
+        if (first) {
+            auto one = [&](uint32_t g, T pn, T q, unsigned m) { sw_[g] = sums(pn, q, pn, inv(g, m), m); };
+            if constexpr (VEC) {
+                pass4<T, KIND, NT, U, ORD>(st, Plain<T>{po}, [&](uint32_t g0, const Vec4<T> &pc, const Vec4<T> &ap,
+                                                               const unsigned (&m)[4]) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (m[k] & ACTIVE) one(g0 + k, pc.v[k], ap.v[k], m[k]);
+                });
+            } else {
+                pass<T, KIND, NT, U, ORD>(st, [&](uint32_t q) { return po[q]; }, [&](uint32_t g, const auto &row) {
+                    one(g, row.pc, product<T, KIND>(st, row), row.m);
+                });
+            }
+        } else {
+            const NextDirection<T> f{zc, so, po, al, bt};
+            if constexpr (VEC) {
+                pass4<T, KIND, NT, U, ORD>(st, f, [&](uint32_t g0, const Vec4<T> &pc, const Vec4<T> &ap,
+                                                     const unsigned (&m)[4]) {
+                    const Vec4<T> zo = ld4(f.z, g0), sv = ld4(f.s, g0), pv = ld4(f.p, g0);
+                    Vec4<double> xv = ld4(x, g0);
+                    Vec4<T> zn, sn, pn = pc;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (!(m[k] & ACTIVE)) {
+                            zn.v[k] = sn.v[k] = pn.v[k] = T(0);
+                            continue;
+                        }
+                        zn.v[k] = nma(al, sv.v[k], zo.v[k]);
+                        sn.v[k] = sums(pc.v[k], ap.v[k], zn.v[k], inv(g0 + k, m[k]), m[k]);
+                        xv.v[k] += xa * (double)pv.v[k];
+                    }
+                    st4(zw, g0, zn);
+                    st4(pw, g0, pn);
+                    st4(sw_, g0, sn);
+                    st4(x, g0, xv);
+                });
+            } else {
+                pass<T, KIND, NT, U, ORD>(st, [&](uint32_t q) { return f.at(q); }, [&](uint32_t g, const auto &row) {
+                    const T zn = nma(al, f.s[g], f.z[g]);
+                    x[g] += xa * (double)f.p[g];
+                    sw_[g] = sums(row.pc, product<T, KIND>(st, row), zn, inv(g, row.m), row.m);
+                    zw[g] = zn;
+                    pw[g] = row.pc;
+                });
+            }
+        }
+        if (!grid_reduce8<NT>(a, v, red)) return;
+        si ^= 1;
+        if (!first) {
+            pi ^= 1;
+            zi ^= 1;
+            zc = bz(zi);
+        }
+        rz = v[5];
+        rr = v[6];
+        alpha = (pre ? rz : rr) / v[0];
+        const double ad = (double)(T)alpha;
+        double rzn = rz - ad * (2.0 * v[1] - ad * v[2]), rrn = rr - ad * (2.0 * v[3] - ad * v[4]);
+        its += 1;
+        updated = false;
+        if (!(rrn > GUARD * rr && rzn > GUARD * rz)) {
+            // the new z itself, and its own sums
+            const T *zo = zc, *s2 = bs(si);
+            T *zn_ = bz(zi ^ 1);
+            const T a2 = (T)alpha;
+            zero();
+            stream([&](uint32_t g, unsigned m) {
+                const T zn = nma(a2, s2[g], zo[g]);
+                const double r = (double)r_of(zn, inv(g, m), m);
+                zn_[g] = zn;
+                v[0] += r * (double)zn;
+                v[1] += r * r;
+            });
+            if (!grid_reduce8<NT>(a, v, red)) return;
+            zi ^= 1;
+            zc = bz(zi);
+            rzn = v[0];
+            rrn = v[1];
+            updated = true;
+        }
+        const bool last = its >= max_its;
+        if (!MIXED) {
+            error = rrn;
+            done = rrn <= tol || last;
+            beta = pre ? rzn / rz : rrn / rr;
+            first = false;
+            if (done) {
+                rz = rzn;
+                rr = rrn;
+                stream([&](uint32_t g, unsigned) { x[g] += alpha * (double)bp(pi)[g]; });
+            }
+        } else if (rrn <= fmax(c->refine_floor, ratio * rr_ref) || last) {
+            // FP64 true residual replaces the FP32 recurrence; restart from it
+            stream([&](uint32_t g, unsigned) { x[g] += alpha * (double)bp(pi)[g]; });
+            zero();
+            if (!grid_reduce8<NT>(a, v, red)) return;
+            t3[0] = t3[1] = t3[2] = 0.0;
+            residual_pass<MIXED, KIND, NT, U, VEC, ORD>(a, bz(zi ^ 1), bp(pi ^ 1), pre, itab, t3);
+            zero();
+            v[0] = t3[0]; v[1] = t3[1]; v[2] = t3[2];
+            if (!grid_reduce8<NT>(a, v, red)) return;
+            pi ^= 1;
+            zc = bp(pi);
+            refinements += 1;
+            error = v[2];
+            rr_ref = v[2];
+            rz = v[0];
+            rr = v[1];
+            first = true;
+            done = error <= tol || last;
+        } else {
+            beta = pre ? rzn / rz : rrn / rr;
+            error = rrn;
+            first = false;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c->its = its;
+        c->error = error;
+        c->refinements = refinements;
+        c->rz = rz;
+        c->rr = rr;
+        c->done = 1;
+    }
+}
+
 // Per-cell code bytes (kinds 0, 1) or class-table row ids (kind 2), built once
 // per operator: bit q of the code says whether face q (-x,+x,-y,+y,-z,+z)
 // couples the cell to an active neighbour inside the domain; bit 6 whether
@@ -707,6 +945,25 @@ static Variant variant(int mixed, int kind, int v) {
     return mixed ? variant_of<true>(kind, v) : variant_of<false>(kind, v);
 }
 
+// Fused form, 7-point operators (kinds 0, 1): one cell per thread, and four-cell groups
+// in both sweeps, one block of 512 threads per SM (fewer arrivals per reduction; shapes
+// with two blocks or 64 registers per thread were slower at every size).
+constexpr int NUM_FUSED = 3;
+#define MB_FUSED(K)                                                         \
+    {(const void *)k_ffcg<MIXED, K, 512, 1, 1, false, 0>, 512, 0, 1},       \
+        {(const void *)k_ffcg<MIXED, K, 512, 1, 1, true, 0>, 512, 1, 1},    \
+        {(const void *)k_ffcg<MIXED, K, 512, 1, 1, true, 1>, 512, 1, 1}
+
+template <bool MIXED>
+static Variant fused_of(int kind, int v) {
+    static const Variant t0[NUM_FUSED] = {MB_FUSED(0)};
+    static const Variant t1[NUM_FUSED] = {MB_FUSED(1)};
+    return kind == 0 ? t0[v] : t1[v];
+}
+#undef MB_FUSED
+
+static Variant fused(int mixed, int kind, int v) { return mixed ? fused_of<true>(kind, v) : fused_of<false>(kind, v); }
+
 }  // namespace fcg
 }  // namespace mb
 
@@ -723,13 +980,27 @@ extern "C" int mbk_fcg_variant_groups(int v) {
 }
 
 // Co-resident blocks of a variant (the grid size of its cooperative launch).
-extern "C" int mbk_fcg_max_blocks(int mixed, int kind, int v) {
+static int max_blocks(const Variant &var) {
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    const Variant var = variant(mixed, kind, v);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, var.fn, var.threads, 0) != cudaSuccess) return -1;
     return sms * per;
+}
+extern "C" int mbk_fcg_max_blocks(int mixed, int kind, int v) { return max_blocks(variant(mixed, kind, v)); }
+
+// The fused form's shapes.
+extern "C" int mbk_ffcg_variants(void) { return NUM_FUSED; }
+extern "C" int mbk_ffcg_variant_groups(int v) { return v >= 0 && v < NUM_FUSED ? fused(0, 0, v).groups : 0; }
+extern "C" int mbk_ffcg_max_blocks(int mixed, int kind, int v) { return max_blocks(fused(mixed, kind, v)); }
+// Whether the fused form is a candidate: a 7-point operator on up to 2^20 cells.  Its gain
+// is a reduction per iteration (2.6 us), its cost the third array gathered at the
+// row's points: per solve 75 against 94 us at 65 k cells (FP64, 13 iterations), 121
+// against 133 at 200 k, 219 against 224 at 576 k, and 174 against 162 us at 1.35 M
+// (mixed, 8 iterations), 381 against 341 at 2 M.  27-point rows gather 19 points: never
+// faster.
+extern "C" int mbk_ffcg_usable(const mb_stencil_dev *st) {
+    return st->kind < 2 && (long long)st->nx * st->ny * st->nz <= (1LL << 20);
 }
 
 extern "C" int mbk_stencil_codes(const mb_stencil_dev *st, uint8_t *code, uint16_t *rowid, cudaStream_t s) {
@@ -757,16 +1028,15 @@ extern "C" int mbk_tune_rhs(double *out, const double *vstar, int64_t n, cudaStr
     return (int)cudaGetLastError();
 }
 
-extern "C" int mbk_fcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
+static int launch(const mb_pcg_dev *p, const Variant &var, cudaStream_t s) {
     Args a;
     a.st = p->st;
     a.x = p->x; a.vstar = p->vstar; a.b = p->b;
     a.r64 = p->r64; a.pa64 = p->pa64; a.pb64 = p->pb64; a.z64 = p->z64;
     a.r32 = p->r32; a.pa32 = p->pa32; a.pb32 = p->pb32; a.z32 = p->z32;
-    a.ap64 = p->ap64; a.ap32 = p->ap32;
+    a.ap64 = p->ap64; a.ap32 = p->ap32; a.ap32b = p->ap32b; a.ap64b = p->ap64b;
     a.inv_diag64 = p->inv_diag64; a.inv_diag32 = p->inv_diag32;
     a.partials = p->partials; a.ctrl = p->ctrl; a.bar = p->bar; a.status = p->status;
-    const Variant var = variant(p->mixed, p->st.kind, p->variant);
     // the arrival counter starts from zero in every launch
     cudaError_t e = cudaMemsetAsync(p->bar, 0, 2 * sizeof(unsigned), s);
     if (e != cudaSuccess) return (int)e;
@@ -792,4 +1062,12 @@ extern "C" int mbk_fcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return (int)cudaLaunchKernelExC(&cfg, var.fn, args);
+}
+
+extern "C" int mbk_fcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
+    return launch(p, variant(p->mixed, p->st.kind, p->variant), s);
+}
+
+extern "C" int mbk_ffcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
+    return launch(p, fused(p->mixed, p->st.kind, p->variant), s);
 }

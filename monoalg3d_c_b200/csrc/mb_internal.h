@@ -192,7 +192,8 @@ typedef struct mb_pcg_dev {
     float *z32;
     double *ap64;            /* A p of the current direction (flat kernel) */
     float *ap32;
-    float *ap32b;            /* second A p buffer (z-march fused pass, mixed) */
+    float *ap32b;            /* second A p buffer (z-march fused pass, flat fused form; mixed) */
+    double *ap64b;           /* the same in FP64 (flat fused form)       */
     const double *inv_diag64;/* Jacobi 1/diag (FP64 form)   */
     const float *inv_diag32; /* Jacobi 1/diag (mixed form)  */
     double *partials;        /* 2 * 8 * blocks + 16 */
@@ -200,7 +201,7 @@ typedef struct mb_pcg_dev {
     unsigned *bar;           /* 2 words, zero at start */
     int *status;             /* 0 = ok; set on a barrier timeout */
     int form;                /* MB_PCG_* */
-    int variant;             /* launch-shape variant of cg_flat.cu */
+    int variant;             /* launch-shape variant of cg_flat.cu (flat or fused form) */
     int tiles_x, tiles_y, zchunk, nchunks;
     /* resident kernel (cg_resident.cu): shape, tile grid and tile size,
      * dynamic shared memory per block */
@@ -217,7 +218,12 @@ typedef struct mb_pcg_dev {
     double *zc_w;           /* A x of the fused solve's last residual (mixed), or NULL */
     void *zc_maps;
 } mb_pcg_dev;
-enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3, MB_PCG_CLUSTER = 4 };
+enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3, MB_PCG_CLUSTER = 4, MB_PCG_FUSED = 5 };
+int mbk_ffcg_variants(void);
+int mbk_ffcg_variant_groups(int variant);
+int mbk_ffcg_max_blocks(int mixed, int kind, int variant);
+int mbk_ffcg_usable(const mb_stencil_dev *st);
+int mbk_ffcg_launch(const mb_pcg_dev *p, cudaStream_t s);
 int mbk_ccg_variants(void);
 int mbk_ccg_usable(const mb_pcg_dev *p, int variant);
 int mbk_ccg_launch(const mb_pcg_dev *p, cudaStream_t s);

@@ -356,7 +356,7 @@ void mb_monodomain_destroy(mb_monodomain *m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     destroy_graphs(m);
     void *bufs[] = {m->d_pb, m->d_ppart, m->d_pb32, m->d_bar, m->d_status, m->d_invd, m->d_invd32, m->d_z, m->d_z32,
-                    m->d_rtrue, m->d_ap, m->d_ap32, m->d_ap32b, m->d_ecg_leads, m->d_ecg_part, m->d_ecg_log,
+                    m->d_rtrue, m->d_ap, m->d_ap32, m->d_ap32b, m->d_apb, m->d_ecg_leads, m->d_ecg_part, m->d_ecg_log,
                     m->d_mask, m->d_cells, m->d_v, m->d_vstar, m->d_r, m->d_p, m->d_r32, m->d_p32,
                     m->d_partials, m->d_sv64, m->d_sv32, m->d_stim_bits, m->d_celltype, m->d_scale,
                     m->d_fx, m->d_fy, m->d_fz, m->d_table, m->d_table32, m->d_code, m->d_rowid, m->d_act,
@@ -435,6 +435,7 @@ static int step_ode(mb_monodomain *m) {
 static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
     switch (q->form) {
     case MB_PCG_CLUSTER: return mbk_ccg_launch(q, s);
+    case MB_PCG_FUSED: return mbk_ffcg_launch(q, s);
     case MB_PCG_TILED: return mbk_tcg_launch(q, s);
     case MB_PCG_RESIDENT: return mbk_rcg_launch(q, s);
     case MB_PCG_ZMARCH: return mbk_zcg_launch(q, s);
@@ -444,16 +445,16 @@ static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
 
 /* Picks the CG kernel: every launch-shape variant of the flat persistent
  * kernel, the 2.5D tiled one, where its tiles fit the resident one, for
- * the 27-point class-table operator every variant of the z-march kernel and,
- * where the vectors fit a cluster's shared memory, every cluster size of the
- * cluster kernel solve one system; V is restored after every trial and the
+ * the 27-point class-table operator every variant of the z-march kernel,
+ * where the vectors fit a cluster's shared memory every cluster size of the
+ * cluster kernel, and the fused flat form's shapes solve one system; V is restored after every trial and the
  * fastest by CUDA events is kept.  The system is the tissue's first one with up to
  * 5 mV of noise on V*, so that it takes as many iterations as a step with
  * wave fronts does (the initial state alone is solved in one or two, which ranks
  * the kernels by their set-up).  A candidate whose warm-up run takes over 1.5
  * times the best is not run again.  MB_CG_VARIANT=<n> forces a choice (n = number of
  * flat variants selects the tiled kernel, n + 1 the resident kernel, n + 2 + v
- * z-march variant v, and after all of those the cluster of 2^v blocks). */
+ * z-march variant v, then the cluster of 2^v blocks, then fused shape v). */
 static int cg_autotune(mb_monodomain *m) {
     if (!m->use_pcg) return MB_OK;
     const int mixed = m->pcg.mixed;
@@ -471,9 +472,11 @@ static int cg_autotune(mb_monodomain *m) {
     const int zmarch = mbk_zcg_usable(&m->st) && m->pcg.zc_maps != NULL;
     const int nzv = mbk_zcg_variants();
     const char *env = getenv("MB_CG_VARIANT");
-    const int ncv = mbk_ccg_variants();
-    /* candidates 0..nv-1 flat, nv tiled, nv+1 resident, nv+2.. z-march, then clusters */
-    int lo = 0, hi = nv + 1 + nzv + ncv;
+    const int ncv = mbk_ccg_variants(), nfv = mbk_ffcg_variants();
+    /* candidates 0..nv-1 flat, nv tiled, nv+1 resident, nv+2.. z-march, then
+     * clusters, then the fused flat form */
+    const int c0 = nv + 2 + nzv, f0 = c0 + ncv;
+    int lo = 0, hi = f0 + nfv - 1;
     if (env) lo = hi = atoi(env);
     double *vsave = NULL, *rhs = NULL;
     if (cudaMalloc((void **)&vsave, (size_t)m->n * sizeof(double)) != cudaSuccess)
@@ -504,9 +507,15 @@ static int cg_autotune(mb_monodomain *m) {
             if (!resident) continue;
             q.form = MB_PCG_RESIDENT;
             q.blocks = q.rc_nbx * q.rc_nby;
-        } else if (cand - nv - 2 >= nzv) {
+        } else if (cand >= f0) {
+            if (cand >= f0 + nfv || !mbk_ffcg_usable(&m->st)) continue;
+            q.form = MB_PCG_FUSED;
+            q.variant = cand - f0;
+            if (mbk_ffcg_variant_groups(q.variant) && (m->desc.nx % 4) != 0) continue;
+            q.blocks = mbk_ffcg_max_blocks(mixed, kind, q.variant);
+        } else if (cand >= c0) {
             q.form = MB_PCG_CLUSTER;
-            q.cc_variant = cand - nv - 2 - nzv;
+            q.cc_variant = cand - c0;
             if (!mbk_ccg_usable(&q, q.cc_variant)) continue;
             q.blocks = 1 << q.cc_variant;
         } else {
@@ -560,14 +569,28 @@ static int cg_autotune(mb_monodomain *m) {
     } else if (bestc == nv + 1) {
         m->pcg.form = MB_PCG_RESIDENT;
         m->pcg.blocks = m->pcg.rc_nbx * m->pcg.rc_nby;
-    } else if (bestc - nv - 2 >= nzv) {
+    } else if (bestc >= f0) {
+        m->pcg.form = MB_PCG_FUSED;
+        m->pcg.variant = bestc - f0;
+        m->pcg.blocks = mbk_ffcg_max_blocks(mixed, kind, m->pcg.variant);
+    } else if (bestc >= c0) {
         m->pcg.form = MB_PCG_CLUSTER;
-        m->pcg.cc_variant = bestc - nv - 2 - nzv;
+        m->pcg.cc_variant = bestc - c0;
         m->pcg.blocks = 1 << m->pcg.cc_variant;
     } else {
         m->pcg.form = MB_PCG_ZMARCH;
         m->pcg.zc_variant = bestc - nv - 2;
         m->pcg.blocks = mbk_zcg_max_blocks(mixed, m->pcg.zc_variant);
+    }
+    if (m->pcg.form != MB_PCG_FUSED && m->d_apb) {
+        cudaFree(m->d_apb);
+        m->d_apb = NULL;
+        m->pcg.ap64b = NULL;
+    }
+    if (m->pcg.form != MB_PCG_FUSED && m->pcg.form != MB_PCG_ZMARCH && m->d_ap32b) {
+        cudaFree(m->d_ap32b);
+        m->d_ap32b = NULL;
+        m->pcg.ap32b = NULL;
     }
     if (m->pcg.form != MB_PCG_RESIDENT && m->d_rtrue) {
         cudaFree(m->d_rtrue);
@@ -842,6 +865,10 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
                 const int b = mbk_fcg_max_blocks(mixed, m->st.kind, v);
                 if (b > maxb) maxb = b;
             }
+            for (int v = 0; mbk_ffcg_usable(&m->st) && v < mbk_ffcg_variants(); ++v) {
+                const int b = mbk_ffcg_max_blocks(mixed, m->st.kind, v);
+                if (b > maxb) maxb = b;
+            }
             const int bt = mbk_tcg_max_blocks(mixed);
             if (bt > maxb) maxb = bt;
             if (mbk_zcg_usable(&m->st))
@@ -862,6 +889,10 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
                 CKK(cudaMemset(m->d_z, 0, (size_t)n * sizeof(double)));
                 ALLOC(m->d_ap, (size_t)n * sizeof(double));
                 CKK(cudaMemset(m->d_ap, 0, (size_t)n * sizeof(double)));
+                if (mbk_ffcg_usable(&m->st)) {
+                    ALLOC(m->d_apb, (size_t)n * sizeof(double));
+                    CKK(cudaMemset(m->d_apb, 0, (size_t)n * sizeof(double)));
+                }
             } else {
                 ALLOC(m->d_pb32, (size_t)n * sizeof(float));
                 CKK(cudaMemset(m->d_pb32, 0, (size_t)n * sizeof(float)));
@@ -869,8 +900,8 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
                 CKK(cudaMemset(m->d_z32, 0, (size_t)n * sizeof(float)));
                 ALLOC(m->d_ap32, (size_t)n * sizeof(float));
                 CKK(cudaMemset(m->d_ap32, 0, (size_t)n * sizeof(float)));
-                if (mbk_zcg_usable(&m->st)) {
-                    /* the z-march fused pass alternates A p between two buffers */
+                if (mbk_zcg_usable(&m->st) || mbk_ffcg_usable(&m->st)) {
+                    /* the fused passes alternate A p between two buffers */
                     ALLOC(m->d_ap32b, (size_t)n * sizeof(float));
                     CKK(cudaMemset(m->d_ap32b, 0, (size_t)n * sizeof(float)));
                 }
@@ -911,6 +942,7 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
             q->r32 = m->d_r32; q->pa32 = m->d_p32; q->pb32 = m->d_pb32;
             q->z64 = m->d_z; q->z32 = m->d_z32;
             q->ap64 = m->d_ap; q->ap32 = m->d_ap32; q->ap32b = m->d_ap32b;
+            q->ap64b = m->d_apb;
             q->partials = m->d_ppart;
             q->inv_diag64 = m->d_invd;
             q->inv_diag32 = m->d_invd32;
@@ -1107,7 +1139,8 @@ int mb_monodomain_tuning(mb_monodomain *m, int *ode_variant, int *cg_blocks, int
                    : m->pcg.form == MB_PCG_TILED ? 100
                    : m->pcg.form == MB_PCG_RESIDENT ? 200
                    : m->pcg.form == MB_PCG_ZMARCH ? 300 + m->pcg.zc_variant
-                   : m->pcg.form == MB_PCG_CLUSTER ? 400 + m->pcg.cc_variant : m->pcg.variant;
+                   : m->pcg.form == MB_PCG_CLUSTER ? 400 + m->pcg.cc_variant
+                   : m->pcg.form == MB_PCG_FUSED ? 500 + m->pcg.variant : m->pcg.variant;
     return MB_OK;
 }
 

@@ -1,5 +1,6 @@
-"""The cluster CG kernel (cg_cluster.cu) at every cluster size against the flat
-persistent kernel: blocks that own a few rows or less than a z-plane (neighbours two
+"""The CG kernels with one reduction per iteration -- the cluster kernel
+(cg_cluster.cu) at every cluster size and the fused flat form (cg_flat.cu) in every
+shape -- against the flat persistent kernel with two: blocks that own a few rows or less than a z-plane (neighbours two
 blocks away), a last block that is partly or wholly empty, removed cells,
 per-cell conductivity, 27-point rows, no preconditioner, and a first step whose
 residual vanishes in one iteration (the recurred sums cancel).
@@ -14,7 +15,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = {"cable": (130, 1, 1), "sheet": (97, 23, 1), "slab": (40, 33, 3), "thick": (24, 20, 9), "ragged": (31, 9, 8)}
+SHAPES = {"cable": (130, 1, 1), "sheet": (97, 23, 1), "slab": (40, 33, 3), "thick": (24, 20, 9), "ragged": (31, 9, 8),
+          "wide": (160, 96, 10)}
 
 
 def _kw(form, nx, ny, nz):
@@ -81,3 +83,30 @@ def test_clusters_match_flat(shape, form, precision):
             assert np.abs(i - i0).max() <= 1, f"cluster of {1 << c}: iterations {i} against {i0}"
             np.testing.assert_allclose(v[ok], v0[ok], rtol=0, atol=1e-5)
     assert ran >= 1
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape,form", [("cable", "iso"), ("sheet", "removed"), ("slab", "iso"), ("slab", "plain"),
+                                        ("thick", "percell"), ("thick", "removed"), ("wide", "removed")])
+def test_fused_shapes_match_flat(shape, form, precision):
+    from monoalg3d_c_b200._lib import lib
+    from monoalg3d_c_b200.monodomain import cg_launch_shapes
+    size = SHAPES[shape]
+    kw = _kw(form, *size)
+    k0, v0, i0 = _run(size, precision, 0, **kw)
+    assert k0 == 0
+    first = cg_launch_shapes() + 2 + lib.mbk_zcg_variants() + lib.mbk_ccg_variants()
+    ok = np.isfinite(v0)
+    for f in range(lib.mbk_ffcg_variants()):
+        k, v, i = _run(size, precision, first + f, **kw)
+        if lib.mbk_ffcg_variant_groups(f) and size[0] % 4:
+            assert k == 0
+            continue
+        assert k == 500 + f
+        assert np.array_equal(ok, np.isfinite(v))
+        if precision == "fp64":
+            assert np.array_equal(i, i0), f"fused shape {f}: iterations {i} against {i0}"
+            np.testing.assert_allclose(v[ok], v0[ok], rtol=1e-8, atol=1e-9)
+        else:
+            assert np.abs(i - i0).max() <= 1, f"fused shape {f}: iterations {i} against {i0}"
+            np.testing.assert_allclose(v[ok], v0[ok], rtol=0, atol=1e-5)
