@@ -93,6 +93,10 @@ struct ZArgs {
     // whole z chunks in turn (the window Q pass's form)
     int balanced;
     FastDiv by_gx, by_ny;          // n / (nx / 4), n / ny
+    // cells per x-row of the tissue.  The vectors' rows are padded to a multiple of
+    // 4 (st.nx): the pads, in the group of the last cell, hold zeros (apply27
+    // leaves zeros there, and every other step keeps them)
+    int nxt;
 };
 
 __host__ __device__ constexpr int r128(int b) { return (b + 127) / 128 * 128; }
@@ -311,17 +315,19 @@ __device__ __forceinline__ void load_row(const double *row, double (&cc)[CROW]) 
 // compiler can issue ahead of the arithmetic (measured faster than skipping
 // the entries that are zero in every row, st.nzmask, in both precisions).
 // All 32 lanes call it together.
-// FACE: some lane of the warp holds a cell on an x face (warp-uniform); its
-// own row's sum runs beside the others in the same entry order, from the
+// A face cell's own row's sum runs beside the others in the same entry order, from the
 // same values (the face cell's neighbours are already in the lane's
 // registers), instead of a pass over shared memory after them.
-template <typename R, int W, bool DENSE, bool FACE>
+// FACE: 0 no lane of the warp holds a cell on an x face (warp-uniform); 1 the low face's
+// cell is the first of its four and the high face's the last; 2 the rows are
+// padded, the high face's cell is any of its four (e) and those after it are pads.
+template <typename R, int W, bool DENSE, int FACE>
 __device__ __forceinline__ V4<R> apply27_rows(const mb_stencil_dev &st, const R *lo, const R *mid, const R *hi,
-                                              const R *ct, int e, int cy, int w, int lane) {
+                                              const R *ct, int e, bool high, int cy, int w, int lane) {
     const R *cm = ct + (cy * 3 + 1) * CROW;
     // the face row of a lane holding a face cell (lanes without one read
     // the low face's row and drop the sum)
-    const R *ce = ct + (cy * 3 + (e == 3 ? 2 : 0)) * CROW;
+    const R *ce = ct + (cy * 3 + (high ? 2 : 0)) * CROW;
     const uint32_t mask = DENSE ? 0x7ffffffu : st.nzmask;
     // FP32: the row in registers, loaded as vectors; FP64 reads each entry
     // where it is used (its 28 values would take 56 registers)
@@ -364,14 +370,25 @@ __device__ __forceinline__ V4<R> apply27_rows(const mb_stencil_dev &st, const R 
                 else cq = cm[q];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[c] = fma(cq, wv[c + 1 + dx], acc[c]);
-                // the face cell (e = 0 or 3) and its neighbours e + dx
-                if constexpr (FACE) af = fma(ce[q], e == 3 ? wv[4 + dx] : wv[1 + dx], af);
+                // the face cell e and its neighbours e + dx
+                if constexpr (FACE == 1) af = fma(ce[q], e == 3 ? wv[4 + dx] : wv[1 + dx], af);
+                if constexpr (FACE == 2) {
+                    const R a = (e & 1) ? wv[2 + dx] : wv[1 + dx], b = (e & 1) ? wv[4 + dx] : wv[3 + dx];
+                    af = fma(ce[q], (e & 2) ? b : a, af);
+                }
             }
         }
     }
-    if constexpr (FACE) {
+    if constexpr (FACE == 1) {
         if (e == 0) acc[0] = af;
         else if (e == 3) acc[3] = af;
+    }
+    if constexpr (FACE == 2) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c == e) acc[c] = af;
+            if (high && c > e) acc[c] = R(0);
+        }
     }
     V4<R> out;
 #pragma unroll
@@ -380,14 +397,22 @@ __device__ __forceinline__ V4<R> apply27_rows(const mb_stencil_dev &st, const R 
 }
 
 template <typename R, int W, bool DENSE = true>
-__device__ __forceinline__ V4<R> apply27(const mb_stencil_dev &st, const R *lo, const R *mid, const R *hi,
+__device__ __forceinline__ V4<R> apply27(const mb_stencil_dev &st, int nxt, const R *lo, const R *mid, const R *hi,
                                          const R *ct, int i0, int j, int w, int lane) {
     const int cy = axis_class(j, st.ny);
-    // the lane's cell on an x face, if any: the first of its four on the
-    // low face, the last on the high face
-    const int e = i0 == 0 ? 0 : (i0 + 3 == st.nx - 1 ? 3 : -1);
-    if (__any_sync(0xffffffffu, e >= 0)) return apply27_rows<R, W, DENSE, true>(st, lo, mid, hi, ct, e, cy, w, lane);
-    return apply27_rows<R, W, DENSE, false>(st, lo, mid, hi, ct, e, cy, w, lane);
+    // the lane's cell on an x face, if any; with whole rows the first of its four on
+    // the low face, the last on the high face
+    if (nxt == st.nx) {
+        const int e = i0 == 0 ? 0 : (i0 + 3 == st.nx - 1 ? 3 : -1);
+        if (__any_sync(0xffffffffu, e >= 0))
+            return apply27_rows<R, W, DENSE, 1>(st, lo, mid, hi, ct, e, e == 3, cy, w, lane);
+        return apply27_rows<R, W, DENSE, 0>(st, lo, mid, hi, ct, e, false, cy, w, lane);
+    }
+    const bool high = i0 < nxt && i0 + 3 >= nxt - 1;
+    const int e = i0 == 0 ? 0 : (high ? nxt - 1 - i0 : -1);
+    if (!__any_sync(0xffffffffu, e >= 0))
+        return apply27_rows<R, W, DENSE, 0>(st, lo, mid, hi, ct, e, high, cy, w, lane);
+    return apply27_rows<R, W, DENSE, 2>(st, lo, mid, hi, ct, e, high, cy, w, lane);
 }
 
 // The 27-point product for the lane's four cells of row j of plane k from a
@@ -617,7 +642,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
     T *bufb = MIXED ? (T *)a.pb32 : (T *)a.pb64;
     T *__restrict__ apb = MIXED ? (T *)a.ap32 : (T *)a.ap64;
     const T *invt = inv_table<T>(z);
-    const int nx = st.nx, ny = st.ny, nz = st.nz;
+    const int nx = st.nx, ny = st.ny, nz = st.nz, nxt = z.nxt;    // nx: padded rows
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
@@ -690,7 +715,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
             V4<double> bv = {{0.0, 0.0, 0.0, 0.0}};
             if (i0 < nx) bv = ld4(a.b ? a.b + g0 : a.vstar + g0);
             const double *ct = tab64 + ts * TSLOT;
-            const V4<double> ax = apply27<double, W>(st, reinterpret_cast<const double *>(lo),
+            const V4<double> ax = apply27<double, W>(st, nxt, reinterpret_cast<const double *>(lo),
                                                      reinterpret_cast<const double *>(mid),
                                                      reinterpret_cast<const double *>(hi), ct, i0, j, w, lane);
             if (i0 >= nx) return;
@@ -701,7 +726,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                 const double bb = a.b ? bv.v[e] : st.alpha * bv.v[e];
                 const double r64 = bb - ax.v[e];
                 const T rt = (T)r64;
-                const T zz = pre ? mul_rn(iv[axis_class(i0 + e, nx)], rt) : rt;
+                const T zz = pre ? mul_rn(iv[axis_class(i0 + e, nxt)], rt) : rt;
                 rv.v[e] = rt;
                 acc[0] += (double)rt * (double)zz;
                 acc[1] += (double)rt * (double)rt;
@@ -738,7 +763,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                 const double bb = a.b ? bv.v[e] : st.alpha * bv.v[e];
                 const double r64 = bb - wv.v[e];
                 const T rt = (T)r64;
-                const T zz = pre ? mul_rn(__ldg(irow + axis_class(i0 + e, nx)), rt) : rt;
+                const T zz = pre ? mul_rn(__ldg(irow + axis_class(i0 + e, nxt)), rt) : rt;
                 rv.v[e] = rt;
                 acc[0] += (double)rt * (double)zz;
                 acc[1] += (double)rt * (double)rt;
@@ -774,11 +799,11 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                 // away from the x faces the four cells share one class
                 const T *irow = itab + axis_class(j, ny) * 3;
                 T iv[4];
-                if (i > 0 && i + 3 < nx - 1) {
+                if (i > 0 && i + 3 < nxt - 1) {
                     iv[0] = iv[1] = iv[2] = iv[3] = irow[1];
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) iv[q] = irow[axis_class(i + q, nx)];
+                    for (int q = 0; q < 4; ++q) iv[q] = irow[axis_class(i + q, nxt)];
                 }
                 V4<T> pv;
 #pragma unroll
@@ -795,7 +820,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
             const int j = U.y0 + w, i0 = U.x0 + 4 * lane;
             if (j >= ny) return;
             const T *pm = reinterpret_cast<const T *>(mid);
-            const V4<T> ap = apply27<T, W>(st, reinterpret_cast<const T *>(lo), pm, reinterpret_cast<const T *>(hi),
+            const V4<T> ap = apply27<T, W>(st, nxt, reinterpret_cast<const T *>(lo), pm, reinterpret_cast<const T *>(hi),
                                            tabT(ts), i0, j, w, lane);
             if (i0 >= nx) return;
             const size_t g0 = (size_t)i0 + (size_t)nx * ((size_t)j + (size_t)ny * k);
@@ -899,11 +924,11 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                     V4<T> po = {{T(0), T(0), T(0), T(0)}};
                     if (!first) po = ld4(ps + o);
                     T iv[4];
-                    if (i0 > 0 && i0 + 3 < nx - 1) {
+                    if (i0 > 0 && i0 + 3 < nxt - 1) {
                         iv[0] = iv[1] = iv[2] = iv[3] = (T)irow[1];
                     } else {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) iv[q] = (T)irow[axis_class(i0 + q, nx)];
+                        for (int q = 0; q < 4; ++q) iv[q] = (T)irow[axis_class(i0 + q, nxt)];
                     }
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -917,7 +942,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                         const int ce = lane == 0 ? -1 : 4;
                         const T re = rs[o + ce];
                         const T pe = first ? T(0) : ps[o + ce];
-                        const T ie = (T)irow[axis_class(i0 + ce, nx)];
+                        const T ie = (T)irow[axis_class(i0 + ce, nxt)];
                         const T zz = pre ? mul_rn(ie, re) : re;
                         ph = first ? zz : fma(bt, pe, zz);
                     }
@@ -998,7 +1023,11 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                     const T lo = __ldg(irow), mi = __ldg(irow + 1), hi = __ldg(irow + 2);
                     iv[0] = i0 == 0 ? lo : mi;
                     iv[1] = iv[2] = mi;
-                    iv[3] = i0 + 3 == nx - 1 ? hi : mi;
+                    iv[3] = i0 + 3 >= nxt - 1 ? hi : mi;
+                    if (nxt != nx && i0 > 0) {
+#pragma unroll
+                        for (int e = 0; e < 3; ++e) iv[e] = i0 + e >= nxt - 1 ? hi : mi;
+                    }
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -1082,11 +1111,11 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                 }
                 const T *irow = itab + axis_class(j, ny) * 3;
                 T iv[4];
-                if (i > 0 && i + 3 < nx - 1) {
+                if (i > 0 && i + 3 < nxt - 1) {
                     iv[0] = iv[1] = iv[2] = iv[3] = irow[1];
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) iv[q] = irow[axis_class(i + q, nx)];
+                    for (int q = 0; q < 4; ++q) iv[q] = irow[axis_class(i + q, nxt)];
                 }
                 V4<T> pv;
 #pragma unroll
@@ -1120,7 +1149,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
             const int j = U.y0 + w, i0 = U.x0 + 4 * lane;
             if (j >= ny) return;
             const T *pm = reinterpret_cast<const T *>(mid);
-            const V4<T> q = apply27<T, W>(st, reinterpret_cast<const T *>(lo), pm, reinterpret_cast<const T *>(hi),
+            const V4<T> q = apply27<T, W>(st, nxt, reinterpret_cast<const T *>(lo), pm, reinterpret_cast<const T *>(hi),
                                           tabT(ts), i0, j, w, lane);
             if (i0 >= nx) return;
             const size_t g0 = (size_t)i0 + (size_t)nx * ((size_t)j + (size_t)ny * k);
@@ -1133,7 +1162,11 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
                 const T *irow = tabT(ts) + JOFF + axis_class(j, ny) * 3;
                 iv[0] = i0 == 0 ? irow[0] : irow[1];
                 iv[1] = iv[2] = irow[1];
-                iv[3] = i0 + 3 == nx - 1 ? irow[2] : irow[1];
+                iv[3] = i0 + 3 >= nxt - 1 ? irow[2] : irow[1];
+                if (nxt != nx && i0 > 0) {
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) iv[e] = i0 + e >= nxt - 1 ? irow[2] : irow[1];
+                }
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -1448,11 +1481,45 @@ extern "C" int mbk_zcg_max_blocks(int mixed, int v) {
     return grid_of(variant(mixed, v));
 }
 
-// Whether the z-march kernel applies: the 27-point class-table operator on a
-// grid whose rows are whole 16-byte vectors (nx % 4 == 0).
+// Whether the z-march kernel applies: the 27-point class-table operator.  Where
+// nx is no multiple of 4 the kernel's vectors have rows padded to one (TMA rows
+// are whole 16-byte vectors), and each solve copies V and V* into padded vectors
+// and V back (48 B per cell, against 48 B per cell and iteration): 1.21 ms per FP64 solve of
+// 254 x 187 x 61 cells and 0.73 ms mixed, where the flat kernel takes 1.72 and 1.57 ms.
 extern "C" int mbk_zcg_usable(const mb_stencil_dev *st) {
-    return st->kind == 2 && st->nx % 4 == 0 && st->nx >= 8 && st->ny >= 1 && st->nz >= 1 && st->table &&
-           st->table32;
+    return st->kind == 2 && st->nx >= 8 && st->ny >= 1 && st->nz >= 1 && st->table && st->table32;
+}
+
+static int padded_nx(const mb_stencil_dev *st) { return (st->nx + 3) & ~3; }
+
+// Cells of the CG vectors of an operator (with the pads where the z-march
+// kernel applies).
+extern "C" int64_t mbk_zcg_cells(const mb_stencil_dev *st) {
+    return (int64_t)(mbk_zcg_usable(st) ? padded_nx(st) : st->nx) * st->ny * st->nz;
+}
+
+// Whether variant v runs on this grid: the window form reads a face cell's
+// neighbours from its own lane only and takes unpadded rows.
+extern "C" int mbk_zcg_variant_usable(const mb_stencil_dev *st, int mixed, int v) {
+    return mbk_zcg_usable(st) && v >= 0 && v < NUM_VARIANTS && variant(mixed, v).fn &&
+           !(variant(mixed, v).mode == QWIN && st->nx % 4 != 0);
+}
+
+// Two vectors of rows of nx cells into rows of np >= nx, the pads zero; and
+// one back.
+__global__ void k_pad(double *x, const double *v, double *b, const double *vstar, int nx, int np, int64_t rows) {
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < rows * np; q += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t row = (uint32_t)q / (uint32_t)np, i = (uint32_t)q - row * (uint32_t)np;
+        const int64_t g = (int64_t)row * nx + i;
+        x[q] = i < (uint32_t)nx ? v[g] : 0.0;
+        b[q] = i < (uint32_t)nx ? vstar[g] : 0.0;
+    }
+}
+__global__ void k_unpad(double *v, const double *x, int nx, int np, int64_t rows) {
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < rows * nx; q += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t row = (uint32_t)q / (uint32_t)nx, i = (uint32_t)q - row * (uint32_t)nx;
+        v[q] = x[(int64_t)row * np + i];
+    }
 }
 
 // Per-plane Jacobi tables (device arrays of nz * 9 values each) and the
@@ -1471,14 +1538,21 @@ extern "C" int mbk_zcg_ptab_floats(void) { return PTAB; }
 // (freed by the tissue).  Called once the CG buffers exist, before any
 // launch or stream capture.  Returns 0 or a CUDA error code.
 extern "C" int mbk_zcg_prepare(mb_pcg_dev *p) {
-    const int nx = p->st.nx, ny = p->st.ny, nz = p->st.nz;
+    const int nx = padded_nx(&p->st), ny = p->st.ny, nz = p->st.nz;
     const int elem = p->mixed ? 4 : 8;
+    if (nx != p->st.nx) {
+        const size_t bytes = (size_t)nx * ny * nz * sizeof(double);
+        cudaError_t e = cudaSuccess;
+        if (!p->zc_xpad) e = cudaMalloc((void **)&p->zc_xpad, bytes);
+        if (e == cudaSuccess && !p->zc_vpad) e = cudaMalloc((void **)&p->zc_vpad, bytes);
+        if (e != cudaSuccess) return (int)e;
+    }
     alignas(64) CUtensorMap tm[NUM_VARIANTS * MAPS];
     memset(tm, 0, sizeof tm);
     const void *bases[MAPS] = {p->mixed ? (const void *)p->r32 : (const void *)p->r64,
                                p->mixed ? (const void *)p->pa32 : (const void *)p->pa64,
                                p->mixed ? (const void *)p->pb32 : (const void *)p->pb64,
-                               (const void *)p->x,
+                               (const void *)(p->zc_xpad ? p->zc_xpad : p->x),
                                p->mixed ? (const void *)p->z32 : nullptr,
                                p->mixed ? (const void *)p->ap32 : nullptr,
                                p->mixed ? (const void *)p->ap32b : nullptr,
@@ -1506,7 +1580,9 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
     if (!var.fn) return (int)cudaErrorInvalidValue;
     // the fused pass alternates r and A p between two buffers each
     if (var.mode == FUSED && (!p->z32 || !p->ap32b)) return (int)cudaErrorInvalidValue;
-    const int nx = p->st.nx, ny = p->st.ny, nz = p->st.nz;
+    const int nx = padded_nx(&p->st), ny = p->st.ny, nz = p->st.nz;
+    const bool ragged = nx != p->st.nx;
+    if (ragged && (var.mode == QWIN || p->b || !p->zc_xpad || !p->zc_vpad)) return (int)cudaErrorInvalidValue;
     const int blocks = p->blocks;
     if (blocks <= 0) return (int)cudaErrorInvalidConfiguration;
     // units: x tiles of 128 cells, y tiles of W rows, z chunks; the number of
@@ -1519,6 +1595,7 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
     z.maps = reinterpret_cast<const CUtensorMap *>(p->zc_maps) + MAPS * p->zc_variant;
     z.tiles_x = (nx + TX - 1) / TX;
     z.tiles_y = (ny + var.warps - 1) / var.warps;
+    z.nxt = p->st.nx;
     z.by_gx = fastdiv((uint32_t)(nx / 4));
     z.by_ny = fastdiv((uint32_t)ny);
     {
@@ -1547,9 +1624,16 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
             else if (!strcmp(env, "balanced")) z.balanced = 1;
         }
     }
-    Args a;
+    Args a{};
     a.st = p->st;
+    a.st.nx = nx;
     a.x = p->x; a.vstar = p->vstar; a.b = p->b;
+    const int64_t rows = (int64_t)ny * nz;
+    if (ragged) {
+        a.x = p->zc_xpad;
+        a.vstar = p->zc_vpad;
+        k_pad<<<1184, 256, 0, s>>>(p->zc_xpad, p->x, p->zc_vpad, p->vstar, p->st.nx, nx, rows);
+    }
     a.r64 = p->r64; a.pa64 = p->pa64; a.pb64 = p->pb64; a.z64 = p->z64;
     a.r32 = p->r32; a.pa32 = p->pa32; a.pb32 = p->pb32; a.z32 = p->z32;
     a.ap64 = p->ap64; a.ap32 = p->ap32; a.ap32b = p->ap32b;
@@ -1574,5 +1658,10 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelExC(&cfg, var.fn, args);
+    e = cudaLaunchKernelExC(&cfg, var.fn, args);
+    if (e == cudaSuccess && ragged) {
+        k_unpad<<<1184, 256, 0, s>>>(p->x, p->zc_xpad, p->st.nx, nx, rows);
+        e = cudaGetLastError();
+    }
+    return (int)e;
 }

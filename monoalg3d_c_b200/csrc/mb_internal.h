@@ -217,6 +217,7 @@ typedef struct mb_pcg_dev {
     float *zc_ptab32;       /* [nz][mbk_zcg_ptab_floats()] per-plane blocks (window Q pass) */
     double *zc_w;           /* A x of the fused solve's last residual (mixed), or NULL */
     void *zc_maps;
+    double *zc_xpad, *zc_vpad; /* x and V* with padded rows (nx no multiple of 4), or NULL */
 } mb_pcg_dev;
 enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3, MB_PCG_CLUSTER = 4, MB_PCG_FUSED = 5 };
 int mbk_ffcg_variants(void);
@@ -242,6 +243,8 @@ int mbk_inv_diag(const mb_stencil_dev *st, double *d64, float *d32, cudaStream_t
 int mbk_zcg_variants(void);
 int mbk_zcg_max_blocks(int mixed, int variant);
 int mbk_zcg_usable(const mb_stencil_dev *st);
+int64_t mbk_zcg_cells(const mb_stencil_dev *st);
+int mbk_zcg_variant_usable(const mb_stencil_dev *st, int mixed, int variant);
 int mbk_zcg_inv_tables(const mb_stencil_dev *st, double *inv64, float *inv32, float *ptab32, cudaStream_t s);
 int mbk_zcg_ptab_floats(void);
 int mbk_zcg_prepare(mb_pcg_dev *p);

@@ -361,7 +361,8 @@ void mb_monodomain_destroy(mb_monodomain *m) {
                     m->d_partials, m->d_sv64, m->d_sv32, m->d_stim_bits, m->d_celltype, m->d_scale,
                     m->d_fx, m->d_fy, m->d_fz, m->d_table, m->d_table32, m->d_code, m->d_rowid, m->d_act,
                     m->d_stim_host, m->d_ctrl, m->d_log, m->d_stim2[0], m->d_stim2[1], m->d_vsnap[0],
-                    m->d_vsnap[1], m->pcg.zc_inv64, m->pcg.zc_inv32, m->pcg.zc_ptab32, m->pcg.zc_maps, m->pcg.zc_w};
+                    m->d_vsnap[1], m->pcg.zc_inv64, m->pcg.zc_inv32, m->pcg.zc_ptab32, m->pcg.zc_maps, m->pcg.zc_w,
+                    m->pcg.zc_xpad, m->pcg.zc_vpad};
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; ++i) cudaFree(bufs[i]);
     for (int i = 0; i < 4; ++i) if (m->ev[i]) cudaEventDestroy(m->ev[i]);
     for (int i = 0; i < 4; ++i)
@@ -519,7 +520,7 @@ static int cg_autotune(mb_monodomain *m) {
             if (!mbk_ccg_usable(&q, q.cc_variant)) continue;
             q.blocks = 1 << q.cc_variant;
         } else {
-            if (!zmarch) continue;
+            if (!zmarch || !mbk_zcg_variant_usable(&m->st, mixed, cand - nv - 2)) continue;
             q.form = MB_PCG_ZMARCH;
             q.zc_variant = cand - nv - 2;
             q.blocks = mbk_zcg_max_blocks(mixed, q.zc_variant);
@@ -591,6 +592,11 @@ static int cg_autotune(mb_monodomain *m) {
         cudaFree(m->d_ap32b);
         m->d_ap32b = NULL;
         m->pcg.ap32b = NULL;
+    }
+    if (m->pcg.form != MB_PCG_ZMARCH) {
+        cudaFree(m->pcg.zc_xpad);
+        cudaFree(m->pcg.zc_vpad);
+        m->pcg.zc_xpad = m->pcg.zc_vpad = NULL;
     }
     if (m->pcg.form != MB_PCG_RESIDENT && m->d_rtrue) {
         cudaFree(m->d_rtrue);
@@ -826,7 +832,8 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
     m->st.rowid = m->d_rowid;
     CKK(mbk_stencil_codes(&m->st, m->d_code, m->d_rowid, m->stream));
 
-    /* CG work vectors */
+    /* CG work vectors (the z-march kernel's rows may be padded) */
+    const int64_t nc = mbk_zcg_cells(&m->st);
     m->cg.precision = d->precision;
     {
         int gb = (int)((n + 255) / 256);
@@ -836,15 +843,15 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
         ALLOC(m->d_partials, (size_t)3 * gb * sizeof(double));
     }
     if (d->precision == MB_PREC_FP64) {
-        ALLOC(m->d_r, (size_t)n * sizeof(double));
-        ALLOC(m->d_p, (size_t)n * sizeof(double));
-        CKK(cudaMemset(m->d_r, 0, (size_t)n * sizeof(double)));
-        CKK(cudaMemset(m->d_p, 0, (size_t)n * sizeof(double)));
+        ALLOC(m->d_r, (size_t)nc * sizeof(double));
+        ALLOC(m->d_p, (size_t)nc * sizeof(double));
+        CKK(cudaMemset(m->d_r, 0, (size_t)nc * sizeof(double)));
+        CKK(cudaMemset(m->d_p, 0, (size_t)nc * sizeof(double)));
     } else {
-        ALLOC(m->d_r32, (size_t)n * sizeof(float));
-        ALLOC(m->d_p32, (size_t)n * sizeof(float));
-        CKK(cudaMemset(m->d_r32, 0, (size_t)n * sizeof(float)));
-        CKK(cudaMemset(m->d_p32, 0, (size_t)n * sizeof(float)));
+        ALLOC(m->d_r32, (size_t)nc * sizeof(float));
+        ALLOC(m->d_p32, (size_t)nc * sizeof(float));
+        CKK(cudaMemset(m->d_r32, 0, (size_t)nc * sizeof(float)));
+        CKK(cudaMemset(m->d_p32, 0, (size_t)nc * sizeof(float)));
     }
     m->cg.x = m->d_v;
     m->cg.vstar = m->d_vstar;
@@ -883,27 +890,27 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
         if (m->use_pcg) {
             const int blocks = maxb;
             if (d->precision == MB_PREC_FP64) {
-                ALLOC(m->d_pb, (size_t)n * sizeof(double));
-                CKK(cudaMemset(m->d_pb, 0, (size_t)n * sizeof(double)));
-                ALLOC(m->d_z, (size_t)n * sizeof(double));
-                CKK(cudaMemset(m->d_z, 0, (size_t)n * sizeof(double)));
-                ALLOC(m->d_ap, (size_t)n * sizeof(double));
-                CKK(cudaMemset(m->d_ap, 0, (size_t)n * sizeof(double)));
+                ALLOC(m->d_pb, (size_t)nc * sizeof(double));
+                CKK(cudaMemset(m->d_pb, 0, (size_t)nc * sizeof(double)));
+                ALLOC(m->d_z, (size_t)nc * sizeof(double));
+                CKK(cudaMemset(m->d_z, 0, (size_t)nc * sizeof(double)));
+                ALLOC(m->d_ap, (size_t)nc * sizeof(double));
+                CKK(cudaMemset(m->d_ap, 0, (size_t)nc * sizeof(double)));
                 if (mbk_ffcg_usable(&m->st)) {
                     ALLOC(m->d_apb, (size_t)n * sizeof(double));
                     CKK(cudaMemset(m->d_apb, 0, (size_t)n * sizeof(double)));
                 }
             } else {
-                ALLOC(m->d_pb32, (size_t)n * sizeof(float));
-                CKK(cudaMemset(m->d_pb32, 0, (size_t)n * sizeof(float)));
-                ALLOC(m->d_z32, (size_t)n * sizeof(float));
-                CKK(cudaMemset(m->d_z32, 0, (size_t)n * sizeof(float)));
-                ALLOC(m->d_ap32, (size_t)n * sizeof(float));
-                CKK(cudaMemset(m->d_ap32, 0, (size_t)n * sizeof(float)));
+                ALLOC(m->d_pb32, (size_t)nc * sizeof(float));
+                CKK(cudaMemset(m->d_pb32, 0, (size_t)nc * sizeof(float)));
+                ALLOC(m->d_z32, (size_t)nc * sizeof(float));
+                CKK(cudaMemset(m->d_z32, 0, (size_t)nc * sizeof(float)));
+                ALLOC(m->d_ap32, (size_t)nc * sizeof(float));
+                CKK(cudaMemset(m->d_ap32, 0, (size_t)nc * sizeof(float)));
                 if (mbk_zcg_usable(&m->st) || mbk_ffcg_usable(&m->st)) {
                     /* the fused passes alternate A p between two buffers */
-                    ALLOC(m->d_ap32b, (size_t)n * sizeof(float));
-                    CKK(cudaMemset(m->d_ap32b, 0, (size_t)n * sizeof(float)));
+                    ALLOC(m->d_ap32b, (size_t)nc * sizeof(float));
+                    CKK(cudaMemset(m->d_ap32b, 0, (size_t)nc * sizeof(float)));
                 }
             }
             ALLOC(m->d_ppart, ((size_t)16 * blocks + 16) * sizeof(double));
@@ -920,7 +927,7 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
                 ALLOC(m->pcg.zc_inv32, (size_t)d->nz * 9 * sizeof(float));
                 ALLOC(m->pcg.zc_ptab32, (size_t)d->nz * mbk_zcg_ptab_floats() * sizeof(float));
                 /* the fused mixed solve's stored A x (its next solve's starting product) */
-                if (d->precision == MB_PREC_MIXED) ALLOC(m->pcg.zc_w, (size_t)n * sizeof(double));
+                if (d->precision == MB_PREC_MIXED) ALLOC(m->pcg.zc_w, (size_t)nc * sizeof(double));
                 CKK(mbk_zcg_inv_tables(&m->st, m->pcg.zc_inv64, m->pcg.zc_inv32, m->pcg.zc_ptab32, m->stream));
             }
             CKK(cudaStreamSynchronize(m->stream));
