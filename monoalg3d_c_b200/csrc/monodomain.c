@@ -452,8 +452,8 @@ static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
  * fastest by CUDA events is kept.  The system is the tissue's first one with up to
  * 5 mV of noise on V*, so that it takes as many iterations as a step with
  * wave fronts does (the initial state alone is solved in one or two, which ranks
- * the kernels by their set-up).  A candidate whose warm-up run takes over 1.5
- * times the best is not run again.  MB_CG_VARIANT=<n> forces a choice (n = number of
+ * the kernels by their set-up).  A candidate's first run is not timed (it may load
+ * the kernel); one whose second takes over 1.2 times the best is not run again.  MB_CG_VARIANT=<n> forces a choice (n = number of
  * flat variants selects the tiled kernel, n + 1 the resident kernel, n + 2 + v
  * z-march variant v, then the cluster of 2^v blocks, then fused shape v). */
 static int cg_autotune(mb_monodomain *m) {
@@ -542,7 +542,7 @@ static int cg_autotune(mb_monodomain *m) {
             float ms = 0;
             cudaEventElapsedTime(&ms, m->ev[0], m->ev[1]);
             if (rep > 0) tsum += ms;      /* first run warms up */
-            else if (ms > 0.75f * best) { tsum = 1e30f; break; }
+            if (rep == 1 && ms > 0.6f * best) { tsum = 1e30f; break; }
         }
         if (!rc && tsum < best) {
             best = tsum;
