@@ -176,6 +176,11 @@ typedef struct mb_csr_dev {
 int mbk_csr_cg_init(const mb_csr_dev *a, mb_ctrl *ctrl, cudaStream_t s);
 int mbk_csr_cg_iter(const mb_csr_dev *a, mb_ctrl *ctrl, cudaStream_t s);
 
+/* the whole solve in one cooperative launch (cg_csr.cu); partials: 16 values per block */
+int mbk_csr_pcg_blocks(int32_t n, int32_t nnz);
+int mbk_csr_pcg(const mb_csr_dev *a, int32_t nnz, int blocks, mb_ctrl *ctrl, double *partials, unsigned *bar, int *status,
+                cudaStream_t s);
+
 int mbk_max_grid_blocks(void);
 
 /* Persistent cooperative CG (one launch per solve). */

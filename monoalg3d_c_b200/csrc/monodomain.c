@@ -1678,13 +1678,17 @@ struct mb_csr {
     int32_t *d_rp, *d_col;
     double *d_val, *d_b, *d_x, *d_r, *d_p, *d_q, *d_id, *d_part;
     mb_ctrl *d_ctrl;
+    unsigned *d_bar;       /* 2 words of the grid barrier, then the status word */
+    int32_t nnz;
+    int blocks;            /* of the cooperative solve */
     cudaStream_t s;
 };
 
 void mb_csr_destroy(mb_csr *m) {
     if (!m) return;
     if (m->s) cudaStreamSynchronize(m->s);
-    void *bufs[] = {m->d_rp, m->d_col, m->d_val, m->d_b, m->d_x, m->d_r, m->d_p, m->d_q, m->d_id, m->d_part, m->d_ctrl};
+    void *bufs[] = {m->d_rp, m->d_col, m->d_val, m->d_b, m->d_x, m->d_r, m->d_p, m->d_q, m->d_id, m->d_part, m->d_ctrl,
+                    m->d_bar};
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; ++i) cudaFree(bufs[i]);
     if (m->s) cudaStreamDestroy(m->s);
     free(m);
@@ -1696,8 +1700,12 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     if (nnz < 0) return set_err(MB_ERR_ARG, "bad row_ptr");
     mb_csr *m = (mb_csr *)calloc(1, sizeof *m);
     if (!m) return set_err(MB_ERR_NOMEM, "out of host memory");
-    int gb = (n + 255) / 256;
-    if (gb > mbk_max_grid_blocks()) gb = mbk_max_grid_blocks();
+    m->nnz = nnz;
+    m->blocks = mbk_csr_pcg_blocks(n, nnz);
+    if (m->blocks < 1) {
+        free(m);
+        return set_err(MB_ERR_CUDA, "mb_csr_create: no device for the cooperative solve");
+    }
     cudaError_t e = cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking);
 #define CSR_ALLOC(p, bytes) if (e == cudaSuccess) e = cudaMalloc((void **)&(p), (bytes))
     CSR_ALLOC(m->d_rp, (size_t)(n + 1) * sizeof(int32_t));
@@ -1709,8 +1717,9 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     CSR_ALLOC(m->d_p, (size_t)n * sizeof(double));
     CSR_ALLOC(m->d_q, (size_t)n * sizeof(double));
     CSR_ALLOC(m->d_id, (size_t)n * sizeof(double));
-    CSR_ALLOC(m->d_part, (size_t)3 * gb * sizeof(double));
+    CSR_ALLOC(m->d_part, (size_t)16 * m->blocks * sizeof(double));
     CSR_ALLOC(m->d_ctrl, sizeof(mb_ctrl));
+    CSR_ALLOC(m->d_bar, 3 * sizeof(unsigned));
 #undef CSR_ALLOC
     if (e == cudaSuccess) e = cudaMemcpy(m->d_rp, row_ptr, (size_t)(n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nnz) e = cudaMemcpy(m->d_col, col, (size_t)nnz * sizeof(int32_t), cudaMemcpyHostToDevice);
@@ -1721,7 +1730,7 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     }
     mb_csr_dev *a = &m->a;
     a->n = n;
-    a->grid_blocks = gb;
+    a->grid_blocks = m->blocks;
     a->row_ptr = m->d_rp; a->col = m->d_col; a->val = m->d_val; a->b = m->d_b; a->x = m->d_x;
     a->r = m->d_r; a->p = m->d_p; a->q = m->d_q; a->inv_diag = m->d_id; a->partials = m->d_part;
     *out = m;
@@ -1740,18 +1749,14 @@ int mb_csr_solve(mb_csr *m, const double *b, double *x, double tolerance, int ma
     c.max_its = max_iterations;
     c.use_precond = use_preconditioner ? 1 : 0;
     CK(cudaMemcpyAsync(m->d_ctrl, &c, sizeof c, cudaMemcpyHostToDevice, m->s));
-    if (mbk_csr_cg_init(&m->a, m->d_ctrl, m->s)) return set_err(MB_ERR_CUDA, "csr init launch failed");
-    for (int it = 0; it < max_iterations + 1; it += 16) {
-        for (int q = 0; q < 16; ++q)
-            if (mbk_csr_cg_iter(&m->a, m->d_ctrl, m->s)) return set_err(MB_ERR_CUDA, "csr iteration launch failed");
-        int32_t done = 0;
-        CK(cudaMemcpyAsync(&done, &m->d_ctrl->done, sizeof done, cudaMemcpyDeviceToHost, m->s));
-        CK(cudaStreamSynchronize(m->s));
-        if (done) break;
-    }
+    CK(cudaMemsetAsync(m->d_bar + 2, 0, sizeof(unsigned), m->s));
+    CKK(mbk_csr_pcg(&m->a, m->nnz, m->blocks, m->d_ctrl, m->d_part, m->d_bar, (int *)(m->d_bar + 2), m->s));
+    unsigned status = 0;
     CK(cudaMemcpyAsync(&c, m->d_ctrl, sizeof c, cudaMemcpyDeviceToHost, m->s));
+    CK(cudaMemcpyAsync(&status, m->d_bar + 2, sizeof status, cudaMemcpyDeviceToHost, m->s));
     CK(cudaMemcpyAsync(x, m->d_x, bytes, cudaMemcpyDeviceToHost, m->s));
     CK(cudaStreamSynchronize(m->s));
+    if (status) return set_err(MB_ERR_CUDA, "CSR CG grid barrier timed out (status %u)", status);
     if (number_of_iterations) *number_of_iterations = (uint32_t)c.its;
     if (error) *error = c.error;
     return MB_OK;
