@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(NT, 1) k_ccg(Args a, uint32_t chunk) {
         c->rz = rz;
         c->rr = rr;
         c->done = 1;
+        if (a.end.on) fcg::step_end(c, a.end);
     }
     cl.sync();        // no block leaves while another may still read its memory
 }
@@ -368,6 +369,7 @@ extern "C" int mbk_ccg_launch(const mb_pcg_dev *p, cudaStream_t s) {
     a.x = p->x; a.vstar = p->vstar; a.b = p->b;
     a.inv_diag64 = p->inv_diag64; a.inv_diag32 = p->inv_diag32;
     a.ctrl = p->ctrl; a.status = p->status;
+    a.end = p->end;
     const int C = 1 << p->cc_variant;
     uint32_t chunk = chunk_of((uint32_t)p->st.nx * p->st.ny * p->st.nz, C);
     void *args[] = {&a, &chunk};

@@ -29,7 +29,29 @@ struct Args {
     mb_ctrl *ctrl;
     unsigned *bar;             // [0] arrivals since launch (zeroed before each launch)
     int *status;
+    mb_step_end end;           // the loop step's end, by the thread that writes the result
 };
+
+// The end of a loop step: the solve's record, the NaN flag, periodic stimuli and
+// the clock (monodomain_solver.c:746,907-908).
+__device__ __forceinline__ void step_end(mb_ctrl *c, const mb_step_end &e) {
+    if (e.log && c->count >= 0 && c->count < e.log_len) {
+        mb_step_stats s;
+        s.cg_iterations = c->its;
+        s.refinements = c->refinements;
+        s.cg_error = c->error;
+        e.log[c->count] = s;
+    }
+    if (isnan(c->error)) c->nan_flag = 1;
+    double time = c->cur_time;
+    for (int j = 0; j < e.num_steps; ++j) time += e.dt_ode;
+    for (int k = 0; k < c->num_stims; ++k) {
+        if (c->stim_period[k] > 0.0 && time >= c->stim_start[k] + c->stim_period[k])
+            c->stim_start[k] = c->stim_start[k] + c->stim_period[k];
+    }
+    c->count += 1;
+    c->cur_time += e.dt_pde;
+}
 
 // Grid-wide sum of NV per-thread values.  Every block reduces its threads
 // (warp shuffles, then one warp over the per-warp sums), stores its partials

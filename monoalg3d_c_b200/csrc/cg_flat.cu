@@ -588,6 +588,7 @@ __global__ void __launch_bounds__(NT, MINB) k_fcg(Args a) {
         c->rz = rz;
         c->rr = rr;
         c->done = 1;
+        if (a.end.on) step_end(c, a.end);
     }
 }
 
@@ -825,6 +826,7 @@ __global__ void __launch_bounds__(NT, MINB) k_ffcg(Args a) {
         c->rz = rz;
         c->rr = rr;
         c->done = 1;
+        if (a.end.on) step_end(c, a.end);
     }
 }
 
@@ -1025,13 +1027,14 @@ extern "C" int mbk_tune_rhs(double *out, const double *vstar, int64_t n, cudaStr
 }
 
 static int launch(const mb_pcg_dev *p, const Variant &var, cudaStream_t s) {
-    Args a;
+    Args a{};
     a.st = p->st;
     a.x = p->x; a.vstar = p->vstar; a.b = p->b;
     a.r64 = p->r64; a.pa64 = p->pa64; a.pb64 = p->pb64; a.z64 = p->z64;
     a.r32 = p->r32; a.pa32 = p->pa32; a.pb32 = p->pb32; a.z32 = p->z32;
     a.ap64 = p->ap64; a.ap32 = p->ap32; a.ap32b = p->ap32b; a.ap64b = p->ap64b;
     a.inv_diag64 = p->inv_diag64; a.inv_diag32 = p->inv_diag32;
+    a.end = p->end;
     a.partials = p->partials; a.ctrl = p->ctrl; a.bar = p->bar; a.status = p->status;
     // the arrival counter starts from zero in every launch
     cudaError_t e = cudaMemsetAsync(p->bar, 0, 2 * sizeof(unsigned), s);

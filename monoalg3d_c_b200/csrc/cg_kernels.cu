@@ -26,6 +26,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "mb_internal.h"
+#include "cg_common.cuh"
 
 namespace mb {
 
@@ -521,25 +522,8 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgm_dir(CgArgs a) {
 // Records the CG result, flags NaN, shifts periodic stimuli
 // (ode_solver.c:225-233) and advances the loop clock
 // (monodomain_solver.c:907-908).
-__global__ void k_step_end(mb_ctrl *c, double dt_pde, double dt_ode, int num_steps, mb_step_stats *log,
-                           int64_t log_len) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (log && c->count >= 0 && c->count < log_len) {
-        mb_step_stats s;
-        s.cg_iterations = c->its;
-        s.refinements = c->refinements;
-        s.cg_error = c->error;
-        log[c->count] = s;
-    }
-    if (isnan(c->error)) c->nan_flag = 1;
-    double time = c->cur_time;
-    for (int j = 0; j < num_steps; ++j) time += dt_ode;
-    for (int k = 0; k < c->num_stims; ++k) {
-        if (c->stim_period[k] > 0.0 && time >= c->stim_start[k] + c->stim_period[k])
-            c->stim_start[k] = c->stim_start[k] + c->stim_period[k];
-    }
-    c->count += 1;
-    c->cur_time += dt_pde;
+__global__ void k_step_end(mb_ctrl *c, mb_step_end e) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) fcg::step_end(c, e);
 }
 
 __global__ void k_set_nan(double *v, const uint8_t *mask, int64_t n) {
@@ -704,9 +688,8 @@ extern "C" int mbk_cg_body(const mb_stencil_dev *st, const mb_cg_dev *cg, mb_ctr
     return (int)cudaGetLastError();
 }
 
-extern "C" int mbk_step_end(mb_ctrl *ctrl, double dt_pde, double dt_ode, int num_steps, mb_step_stats *log,
-                            int64_t log_len, cudaStream_t s) {
-    k_step_end<<<1, 32, 0, s>>>(ctrl, dt_pde, dt_ode, num_steps, log, log_len);
+extern "C" int mbk_step_end(mb_ctrl *ctrl, const mb_step_end *e, cudaStream_t s) {
+    k_step_end<<<1, 32, 0, s>>>(ctrl, *e);
     return (int)cudaGetLastError();
 }
 

@@ -1268,6 +1268,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
             // when it was valid and x did not move
             c->w_valid = (a.w != nullptr && (refinements > 1 || wv)) ? 1 : 0;
             c->done = 1;
+            if (a.end.on) fcg::step_end(c, a.end);
         }
         return;
     }
@@ -1339,6 +1340,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_zcg(Args a, ZArgs z) {
         c->rr = rr;
         c->w_valid = 0;          // x moved without the fused solve's product
         c->done = 1;
+        if (a.end.on) fcg::step_end(c, a.end);
     }
 }
 
@@ -1644,6 +1646,7 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
         if (env && !strcmp(env, "0")) a.w = nullptr;
     }
     a.inv_diag64 = p->inv_diag64; a.inv_diag32 = p->inv_diag32;
+    a.end = p->end;
     a.partials = p->partials; a.ctrl = p->ctrl; a.bar = p->bar; a.status = p->status;
     cudaError_t e = cudaMemsetAsync(p->bar, 0, 2 * sizeof(unsigned), s);
     if (e != cudaSuccess) return (int)e;

@@ -155,12 +155,19 @@ typedef struct mb_cg_dev {
     const double *b;     /* explicit right-hand side (CSR path) or NULL       */
 } mb_cg_dev;
 
+/* The end of a loop step (k_step_end), done by the solve's kernel itself. */
+typedef struct mb_step_end {
+    int32_t on, num_steps;
+    double dt_pde, dt_ode;
+    mb_step_stats *log;
+    int64_t log_len;
+} mb_step_end;
+
 int mbk_cg_init(const mb_stencil_dev *st, const mb_cg_dev *cg, mb_ctrl *ctrl,
                 unsigned long long cond, int use_cond, cudaStream_t s);
 int mbk_cg_body(const mb_stencil_dev *st, const mb_cg_dev *cg, mb_ctrl *ctrl,
                 unsigned long long cond, int use_cond, cudaStream_t s);
-int mbk_step_end(mb_ctrl *ctrl, double dt_pde, double dt_ode, int num_steps,
-                 mb_step_stats *log, int64_t log_len, cudaStream_t s);
+int mbk_step_end(mb_ctrl *ctrl, const struct mb_step_end *e, cudaStream_t s);
 int mbk_set_nan(double *v, const uint8_t *mask, int64_t n, cudaStream_t s);
 
 /* CSR CG (general matrices). */
@@ -222,6 +229,7 @@ typedef struct mb_pcg_dev {
     float *zc_ptab32;       /* [nz][mbk_zcg_ptab_floats()] per-plane blocks (window Q pass) */
     double *zc_w;           /* A x of the fused solve's last residual (mixed), or NULL */
     void *zc_maps;
+    mb_step_end end;         /* flat, fused, cluster and z-march kernels        */
     double *zc_xpad, *zc_vpad; /* x and V* with padded rows (nx no multiple of 4), or NULL */
 } mb_pcg_dev;
 enum { MB_PCG_FLAT = 0, MB_PCG_TILED = 1, MB_PCG_RESIDENT = 2, MB_PCG_ZMARCH = 3, MB_PCG_CLUSTER = 4, MB_PCG_FUSED = 5 };

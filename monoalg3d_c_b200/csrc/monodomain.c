@@ -1166,9 +1166,36 @@ static int cap_cginit(mb_monodomain *m, int in_body) {
     return mbk_cg_init(&m->st, &m->cg, m->d_ctrl, 0ULL, 0, m->stream);
 }
 
+static mb_step_end step_end_of(const mb_monodomain *m) {
+    mb_step_end e;
+    e.on = 1;
+    e.num_steps = m->num_steps;
+    e.dt_pde = m->desc.dt_pde;
+    e.dt_ode = m->desc.dt_ode;
+    e.log = m->d_log;
+    e.log_len = m->log_len;
+    return e;
+}
+
+static int enqueue_step_end(mb_monodomain *m) {
+    const mb_step_end e = step_end_of(m);
+    return mbk_step_end(m->d_ctrl, &e, m->stream);
+}
+
+/* A persistent solve and the end of the loop step, which the solve's last thread
+ * does where its kernel can (one launch, about 3 us, fewer per step). */
+static int pcg_and_end(mb_monodomain *m) {
+    mb_pcg_dev q = m->pcg;
+    const int own = q.form == MB_PCG_FLAT || q.form == MB_PCG_FUSED || q.form == MB_PCG_CLUSTER || q.form == MB_PCG_ZMARCH;
+    if (own) q.end = step_end_of(m);
+    int e = pcg_launch(&q, m->stream);
+    if (!e && !own) e = enqueue_step_end(m);
+    return e;
+}
+
 static int cap_post(mb_monodomain *m, int in_body) {
     (void)in_body;
-    return mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream);
+    return enqueue_step_end(m);
 }
 
 /* The CG body captured into the conditional node's body graph, given the
@@ -1231,8 +1258,7 @@ static int build_loop_graph(mb_monodomain *m, capture_fn pre, capture_fn post, c
 static int cap_pcg_step(mb_monodomain *m, int in_body) {
     (void)in_body;
     int e = step_ode(m);
-    if (!e) e = pcg_launch(&m->pcg, m->stream);
-    if (!e) e = mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream);
+    if (!e) e = pcg_and_end(m);
     return e;
 }
 
@@ -1286,16 +1312,25 @@ static int cg_enqueue(mb_monodomain *m) {
     return cg_host_loop(m);
 }
 
+/* One CG solve and the end of the loop step. */
+static int cg_and_end(mb_monodomain *m) {
+    if (m->use_pcg) {
+        CKK(pcg_and_end(m));
+        return MB_OK;
+    }
+    int rc = cg_enqueue(m);
+    if (rc) return rc;
+    CKK(enqueue_step_end(m));
+    return MB_OK;
+}
+
 static int step_once(mb_monodomain *m) {
     if (m->use_graphs) {
         CK(cudaGraphLaunch(m->ge_step, m->stream));
         return MB_OK;
     }
     CKK(step_ode(m));
-    int rc = cg_enqueue(m);
-    if (rc) return rc;
-    CKK(mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream));
-    return MB_OK;
+    return cg_and_end(m);
 }
 
 int mb_monodomain_step(mb_monodomain *m, int n) {
@@ -1367,7 +1402,7 @@ int mb_conjugate_gradient(mb_monodomain *m, uint32_t *its, double *error) {
 int mb_advance_time(mb_monodomain *m) {
     if (!m) return set_err(MB_ERR_ARG, "null");
     if (m->phase != 3) return set_err(MB_ERR_STATE, "advance_time before conjugate_gradient");
-    CKK(mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream));
+    CKK(enqueue_step_end(m));
     m->phase = 0;
     return MB_OK;
 }
@@ -1383,10 +1418,9 @@ int mb_monodomain_step_host(mb_monodomain *m, const double *stim_host, double *v
     if (m->use_ecg) CKK(mbk_ecg(&m->st, m->d_v, &m->ecg, m->d_ctrl, m->stream));
     CKK(mbk_ode_step(&o, m->d_ctrl, m->d_v, m->d_vstar, m->stream));
     {
-        int rc = cg_enqueue(m);
+        int rc = cg_and_end(m);
         if (rc) return rc;
     }
-    CKK(mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream));
     if (v_host) {
         CK(cudaMemcpyAsync(v_host, m->d_v, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToHost, m->stream));
         CK(cudaStreamSynchronize(m->stream));
@@ -1441,9 +1475,8 @@ int mb_monodomain_step_host_async(mb_monodomain *m, const double *stim_host, dou
     if (m->use_ecg) CKK(mbk_ecg(&m->st, m->d_v, &m->ecg, m->d_ctrl, m->stream));
     CKK(mbk_ode_step(&o, m->d_ctrl, m->d_v, m->d_vstar, m->stream));
     CK(cudaEventRecord(m->hev[HEV_ODE][s], m->stream));
-    rc = cg_enqueue(m);
+    rc = cg_and_end(m);
     if (rc) return rc;
-    CKK(mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream));
     if (v_host) {
         CK(cudaMemcpyAsync(m->d_vsnap[s], m->d_v, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream));
         CK(cudaEventRecord(m->hev[HEV_VREADY][s], m->stream));
@@ -1650,7 +1683,7 @@ int mb_monodomain_profile_steps(mb_monodomain *m, int n, double *ode_ms, double 
             if (rc) return rc;
         }
         CK(cudaEventRecord(m->ev[2], m->stream));
-        CKK(mbk_step_end(m->d_ctrl, m->desc.dt_pde, m->desc.dt_ode, m->num_steps, m->d_log, m->log_len, m->stream));
+        CKK(enqueue_step_end(m));
         CK(cudaEventRecord(m->ev[3], m->stream));
         CK(cudaEventSynchronize(m->ev[3]));
         float a = 0, b = 0, c = 0;
