@@ -119,6 +119,8 @@ struct mb_ode {
     mb_ode_dev dev;
     int neq;
     double *d_stim;
+    double *d_dense;       /* the state as neq rows of n, for get / set_state: made at the first
+                              call and kept up to MB_DENSE_KEPT bytes */
     cudaStream_t stream;
 };
 
@@ -159,6 +161,7 @@ void mb_ode_destroy(mb_ode *o) {
     cudaFree(o->dev.sv64);
     cudaFree(o->dev.sv32);
     cudaFree(o->d_stim);
+    cudaFree(o->d_dense);
     if (o->stream) cudaStreamDestroy(o->stream);
     free(o);
 }
@@ -230,27 +233,33 @@ int mb_solve_model_odes_gpu(mb_ode *o, double current_t, const double *stim_curr
     return MB_OK;
 }
 
+#define MB_DENSE_KEPT ((size_t)256 << 20)
+
+static void dense_done(mb_ode *o) {
+    if ((size_t)o->neq * o->dev.n * sizeof(double) <= MB_DENSE_KEPT) return;
+    cudaFree(o->d_dense);
+    o->d_dense = NULL;
+}
+
 int mb_ode_get_state(mb_ode *o, double *host_state) {
     if (!o || !host_state) return set_err(MB_ERR_ARG, "null argument");
-    double *d = NULL;
     const size_t bytes = (size_t)o->neq * o->dev.n * sizeof(double);
-    CK(cudaMalloc((void **)&d, bytes));
-    CKK(mbk_ode_gather(&o->dev, NULL, d, o->stream));
-    CK(cudaMemcpyAsync(host_state, d, bytes, cudaMemcpyDeviceToHost, o->stream));
+    if (!o->d_dense) CK(cudaMalloc((void **)&o->d_dense, bytes));
+    CKK(mbk_ode_gather(&o->dev, NULL, o->d_dense, o->stream));
+    CK(cudaMemcpyAsync(host_state, o->d_dense, bytes, cudaMemcpyDeviceToHost, o->stream));
     CK(cudaStreamSynchronize(o->stream));
-    cudaFree(d);
+    dense_done(o);
     return MB_OK;
 }
 
 int mb_ode_set_state(mb_ode *o, const double *host_state) {
     if (!o || !host_state) return set_err(MB_ERR_ARG, "null argument");
-    double *d = NULL;
     const size_t bytes = (size_t)o->neq * o->dev.n * sizeof(double);
-    CK(cudaMalloc((void **)&d, bytes));
-    CK(cudaMemcpyAsync(d, host_state, bytes, cudaMemcpyHostToDevice, o->stream));
-    CKK(mbk_ode_scatter(&o->dev, d, NULL, o->stream));
+    if (!o->d_dense) CK(cudaMalloc((void **)&o->d_dense, bytes));
+    CK(cudaMemcpyAsync(o->d_dense, host_state, bytes, cudaMemcpyHostToDevice, o->stream));
+    CKK(mbk_ode_scatter(&o->dev, o->d_dense, NULL, o->stream));
     CK(cudaStreamSynchronize(o->stream));
-    cudaFree(d);
+    dense_done(o);
     return MB_OK;
 }
 
