@@ -36,7 +36,8 @@ int mbk_adj_face_grad(const mb_stencil_dev *st, const double *sigma, const doubl
                       double mx, double my, double mz, double *gsig, cudaStream_t s);
 int mbk_adj_gather(const double *v, const int64_t *cells, int ns, double *out, cudaStream_t s);
 int mbk_adj_scatter(double *lam, const int64_t *cells, int ns, const double *gsrc, cudaStream_t s);
-int mbk_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c, cudaStream_t s);
+int mbk_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c, double *part, cudaStream_t s);
+size_t mbk_adj_tol_bytes(void);
 
 struct mb_adjoint {
     mb_monodomain *m;
@@ -49,6 +50,7 @@ struct mb_adjoint {
     double *d_g;           /* nsamples x ns sampled gradients */
     double *d_lam, *d_lam2, *d_w, *d_mu, *d_mu2, *d_gsig, *d_gth, *d_sigma;
     mb_ctrl *d_actrl;      /* control block of the transposed solves */
+    double *d_tolpart;     /* partial sums of their tolerance */
     double alpha, mx, my, mz;
     int have_forward;
 };
@@ -68,7 +70,8 @@ struct mb_adjoint {
 void mb_adjoint_destroy(mb_adjoint *a) {
     if (!a) return;
     void *bufs[] = {a->d_sensors, a->d_ckpt, a->d_seg, a->d_traces, a->d_g, a->d_lam, a->d_lam2, a->d_w, a->d_mu,
-                    a->d_mu2, a->d_gsig, a->d_gth, a->d_sigma, a->d_actrl};
+                    a->d_mu2, a->d_gsig, a->d_gth, a->d_sigma, a->d_actrl,
+                    a->d_tolpart};
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; ++i) cudaFree(bufs[i]);
     mb_monodomain_destroy(a->m);
     free(a);
@@ -119,9 +122,11 @@ int mb_adjoint_create(mb_adjoint **out, const mb_monodomain_desc *d, int nsteps,
     AALLOC(a->d_gth, ld * sizeof(double));
     AALLOC(a->d_sigma, nb);
     AALLOC(a->d_actrl, sizeof(mb_ctrl));
+    AALLOC(a->d_tolpart, mbk_adj_tol_bytes());
 #undef AALLOC
     if (e == cudaSuccess)
         e = cudaMemcpy(a->d_sensors, sensor_cells, (size_t)n_sensors * sizeof(int64_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(a->d_tolpart, 0, mbk_adj_tol_bytes());
     if (e == cudaSuccess) e = cudaMemcpy(a->d_sigma, d->sigma_cell, nb, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         mb_adjoint_destroy(a);
@@ -216,7 +221,7 @@ int mb_adjoint_backward(mb_adjoint *a, const double *dtraces, double *grad_sigma
             mb_tissue_snapshot_parts(m, a->d_seg + a->snap * (size_t)(k + 1), &v1, NULL, NULL);
             mb_tissue_snapshot_parts(m, snap0, &v0, &sv0, NULL);
             /* A w = lambda_{step+1} (warm start from the previous w) */
-            AKK(mbk_adj_tol(a->d_lam, n, 1e-24, a->d_actrl, s));
+            AKK(mbk_adj_tol(a->d_lam, n, 1e-24, a->d_actrl, a->d_tolpart, s));
             AKK(q.form == MB_PCG_CLUSTER ? mbk_ccg_launch(&q, s)
                 : q.form == MB_PCG_FUSED ? mbk_ffcg_launch(&q, s) : mbk_fcg_launch(&q, s));
             /* conductivity gradient through A(sigma) at v_{step+1} */

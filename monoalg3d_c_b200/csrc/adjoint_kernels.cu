@@ -367,22 +367,55 @@ __global__ void k_adj_scatter(double *lam, const int64_t *cells, int ns, const d
     if (i < ns) atomicAdd(&lam[cells[i]], gsrc[i]);
 }
 
-// tol of the transposed solve: rel^2 x (lambda . lambda) (one block, fixed
-// summation order), floored so that an all-zero right-hand side stops at once.
-__global__ void k_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c) {
-    __shared__ double sm[32];
+// tol of the transposed solve: rel^2 x (lambda . lambda), floored so that an all-zero
+// right-hand side stops at once.  Every block leaves its partial sum, the last one
+// to finish adds them in block order (part: TOL_BLOCKS values and, after them, the
+// arrival count, zero between calls).  One block alone took 13 us on 65 k cells.
+constexpr int TOL_BLOCKS = 64;
+
+__global__ void __launch_bounds__(256) k_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c, double *part) {
+    __shared__ double sm[8];
+    __shared__ bool last;
+    unsigned *count = reinterpret_cast<unsigned *>(part + TOL_BLOCKS);
     double s = 0.0;
-    for (int64_t g = threadIdx.x; g < n; g += blockDim.x) s += lam[g] * lam[g];
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (int64_t)gridDim.x * blockDim.x)
+        s += lam[g] * lam[g];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) c->tol = c->refine_floor = fmax(rel2 * s, 1e-300);
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += sm[w];
+        part[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    s = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) s += __ldcg(part + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) {
+        *count = 0;
+        c->tol = c->refine_floor = fmax(rel2 * s, 1e-300);
+    }
+}
+
+// A snapshot of the loop state, or one put back: up to four arrays of 16-byte
+// words in one launch (a copy each cost a launch each).
+struct CopyList {
+    const uint4 *src[4];
+    uint4 *dst[4];
+    int64_t words[4];
+};
+__global__ void __launch_bounds__(256) k_copy4(CopyList l) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        for (int64_t i = t0; i < l.words[q]; i += step) l.dst[q][i] = l.src[q][i];
 }
 
 MB_NS_END
@@ -422,7 +455,27 @@ extern "C" int mbk_adj_scatter(double *lam, const int64_t *cells, int ns, const 
     return (int)cudaGetLastError();
 }
 
-extern "C" int mbk_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c, cudaStream_t s) {
-    k_adj_tol<<<1, 1024, 0, s>>>(lam, n, rel2, c);
+extern "C" size_t mbk_adj_tol_bytes(void) { return (TOL_BLOCKS + 1) * sizeof(double); }
+
+extern "C" int mbk_adj_tol(const double *lam, int64_t n, double rel2, mb_ctrl *c, double *part, cudaStream_t s) {
+    k_adj_tol<<<TOL_BLOCKS, 256, 0, s>>>(lam, n, rel2, c, part);
+    return (int)cudaGetLastError();
+}
+
+// Copies of `arrays` (at most 4) device arrays, each 16-byte aligned and a multiple of
+// 16 bytes long.
+extern "C" int mbk_copy4(int arrays, void *const *dst, const void *const *src, const size_t *bytes, cudaStream_t s) {
+    CopyList l{};
+    int64_t most = 0;
+    for (int q = 0; q < arrays && q < 4; ++q) {
+        l.dst[q] = (uint4 *)dst[q];
+        l.src[q] = (const uint4 *)src[q];
+        l.words[q] = (int64_t)(bytes[q] / 16);
+        if (l.words[q] > most) most = l.words[q];
+    }
+    if (!most) return 0;
+    int64_t blocks = (most + 1023) / 1024;      // four words of the longest array per thread
+    if (blocks > 1184) blocks = 1184;
+    k_copy4<<<(unsigned)blocks, 256, 0, s>>>(l);
     return (int)cudaGetLastError();
 }

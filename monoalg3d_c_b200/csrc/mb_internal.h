@@ -168,6 +168,8 @@ int mbk_cg_init(const mb_stencil_dev *st, const mb_cg_dev *cg, mb_ctrl *ctrl,
 int mbk_cg_body(const mb_stencil_dev *st, const mb_cg_dev *cg, mb_ctrl *ctrl,
                 unsigned long long cond, int use_cond, cudaStream_t s);
 int mbk_step_end(mb_ctrl *ctrl, const struct mb_step_end *e, cudaStream_t s);
+/* up to 4 device arrays (16-byte aligned, whole 16-byte words) copied in one launch */
+int mbk_copy4(int arrays, void *const *dst, const void *const *src, const size_t *bytes, cudaStream_t s);
 int mbk_set_nan(double *v, const uint8_t *mask, int64_t n, cudaStream_t s);
 
 /* CSR CG (general matrices). */

@@ -1848,13 +1848,27 @@ int mb_tissue_snapshot(mb_monodomain *m, void *dev, int restore) {
     size_t off[5], len[5];
     snapshot_layout(m, off, len);
     void *live[5] = {m->d_v, m->d_vstar, m->d_sv64, m->d_sv32, m->d_ctrl};
+    /* the arrays that are whole 16-byte words in one launch, the others by copies */
+    void *dst[4];
+    const void *src[4];
+    size_t bytes[4];
+    int some = 0;
     for (int q = 0; q < 5; ++q) {
         if (!len[q] || !live[q]) continue;
         char *snap = (char *)dev + off[q];
-        cudaError_t e = restore ? cudaMemcpyAsync(live[q], snap, len[q], cudaMemcpyDeviceToDevice, m->stream)
-                                : cudaMemcpyAsync(snap, live[q], len[q], cudaMemcpyDeviceToDevice, m->stream);
+        void *to = restore ? live[q] : snap;
+        const void *from = restore ? (const void *)snap : live[q];
+        if (some < 4 && len[q] % 16 == 0 && ((uintptr_t)to | (uintptr_t)from) % 16 == 0) {
+            dst[some] = to;
+            src[some] = from;
+            bytes[some++] = len[q];
+            continue;
+        }
+        cudaError_t e = cudaMemcpyAsync(to, from, len[q], cudaMemcpyDeviceToDevice, m->stream);
         if (e != cudaSuccess) return set_err(MB_ERR_CUDA, "snapshot copy: %s", cudaGetErrorString(e));
     }
+    const int e = mbk_copy4(some, dst, src, bytes, m->stream);
+    if (e) return set_err(MB_ERR_CUDA, "snapshot copy: %s", cudaGetErrorString((cudaError_t)e));
     if (restore) forget_stored_product(m);
     return MB_OK;
 }
