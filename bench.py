@@ -185,13 +185,11 @@ PROFILED_CG_TRAFFIC = {
 #   (workload, "mixed" | "fp64", ode variant) -> pipe utilisation and MUFU
 #   (XU pipe) warp instructions x 32 per cell-step of one launch
 PROFILED_ODE = {
-    # k_torord_mixed<0, 4> / k_torord_fp64<0, 3> on the 0.72-scale slab
-    ("slab_500x500x100_torord_rotating_fibres", "mixed", 3): {
-        "xu_pct": 48.9, "fma_pct": 34.7, "fp64_pct": 1.2, "dram_bytes_per_cell_step": 411.7,
-        "mufu_per_cell_step": 227.0},
-    ("slab_500x500x100_torord_rotating_fibres", "fp64", 2): {
-        "fp64_pipe_pct": 17.2, "xu_pct": 4.4, "issue_active_pct": 20.6, "fp64_ops_per_cell_step": 3912.0,
-        "mufu_per_cell_step": 248.3},
+    # k_torord_mixed_slots<0, 6> / k_torord_fp64<0, 6> on the 0.72-scale slab
+    ("slab_500x500x100_torord_rotating_fibres", "mixed", 4): {
+        "fma_pct": 38.2, "issue_active_pct": 64.0, "dram_bytes_per_cell_step": 411.5, "mufu_per_cell_step": 196.0},
+    ("slab_500x500x100_torord_rotating_fibres", "fp64", 5): {
+        "fp64_pipe_pct": 52.2, "issue_active_pct": 56.3, "fp64_ops_per_cell_step": 2132.0, "mufu_per_cell_step": 95.3},
 }
 
 
@@ -581,7 +579,9 @@ def main():
                 "d2h_bytes_per_step": n_grid * 8, "timed_blocks_ms": e2e_blocks,
                 "call": "mb_monodomain_step_host_async (copies of every step overlapped with the next steps)",
                 "synchronous": {"value": e2e_sync, "call": "mb_monodomain_step_host (copy in, step, copy out, wait)"}},
-        "gpu_launches": 3 * args.steps * args.repeats,
+        # the cell models and the solve, whose kernel ends the step (the tiled and
+        # resident forms leave that to a third launch)
+        "gpu_launches": (3 if cg_kernel in (-1, 100, 200) else 2) * args.steps * args.repeats,
         "clocks": clk_mx,
     }
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
