@@ -501,7 +501,9 @@ static int cg_autotune(mb_monodomain *m) {
     cudaMemcpyAsync(vsave, m->d_v, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
     float best = 1e30f;
     int bestc = 0, rc = MB_OK;      /* variant 0 runs on every grid */
-    for (int cand = lo; cand <= hi && !rc; ++cand) {
+    /* the specialised kernels first: where one applies it is the faster, and the
+     * others then end after their second run */
+    for (int cand = hi; cand >= lo && !rc; --cand) {
         mb_pcg_dev q = m->pcg;
         if (rhs) q.vstar = rhs;
         if (cand < nv) {
