@@ -68,8 +68,9 @@ __device__ __forceinline__ void exp_table_fill() {
 // 2^(n/128) (1 + r + r^2/2 + ... + r^5/120), n = 128 k + j; the first omitted
 // term is below 6e-19.  Arguments beyond +-700 are taken as +-700 (1e304, far
 // from every value a rate of the models can still tell from infinity, so no
-// denominator overflows).  So is NaN: a state that is NaN makes dV/dt NaN
-// through the terms outside the exponentials.
+// denominator overflows).  NaN gives NaN: a concentration that has left its range
+// (the logarithm or root of a negative value) reaches V through exponentials
+// alone.  Its test is on the scale's side, off the chain through r.
 __device__ __forceinline__ double mexp(double x) {
     const int hi = __double2hiint(x);
     x = __hiloint2double(min(hi & 0x7fffffff, 0x4085e000) | (hi & (int)0x80000000), __double2loint(x));   // 700.0
@@ -83,7 +84,8 @@ __device__ __forceinline__ double mexp(double x) {
     q = fma(q, r, 1.0 / 6.0);
     q = fma(q, r, 0.5);
     const double p = fma(r * r, q, r + row.y);
-    const double s = __hiloint2double(__double2hiint(row.x) + n * 8192, __double2loint(row.x));
+    const bool nan = (hi & 0x7fffffff) > 0x7ff00000;
+    const double s = __hiloint2double(nan ? 0x7ff80000 : __double2hiint(row.x) + n * 8192, __double2loint(row.x));
     return fma(s, p, s);
 }
 

@@ -42,6 +42,7 @@ def test_exponential_outside():
     got = _eval(0, np.array([701.0, 1e5, 1e300, np.inf, -701.0, -1e5, -1e300, -np.inf]))
     assert (got[:4] >= np.exp(699.99)).all() and (got[:4] <= np.exp(700.07)).all()
     assert (got[4:] <= np.exp(-699.99)).all() and (got[4:] >= np.exp(-700.07)).all()
+    assert np.isnan(_eval(0, np.array([np.nan, -np.nan]))).all()
 
 
 def test_reciprocal_and_quotient():

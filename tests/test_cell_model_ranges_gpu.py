@@ -1,0 +1,59 @@
+"""One step of the GPU cell models (mb_ode) from states outside their usual range
+against the oracle's step: a model written with other quotients and its own
+exponential has to be finite, and not a number, where the reference's formulas
+are.
+
+Bars, where a value is finite: FP64 1e-9 relative (a step is a few hundred roundings);
+mixed 1e-3 relative (hardware exponentials, 1e-5 at arguments near 85)."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oracle"))
+import oracle  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+DT = 0.02
+
+
+def _steps(model, precision, states):
+    """(product, oracle) states after one step of every column of states."""
+    from monoalg3d_c_b200 import OdeSolver
+    n = states.shape[1]
+    s = OdeSolver(model, n, DT, precision=precision)
+    s.set_model_initial_conditions_gpu()
+    s.set_state(states)
+    s.solve_model_odes_gpu(1.0)
+    got = s.state()
+    s.close()
+    ref = np.ascontiguousarray(states.T).copy()
+    L = oracle.load()
+    for row in ref:
+        if model == "tt2006":
+            L.orc_tt2006_step(row.ctypes.data, 0.0, DT, None)
+        else:
+            L.orc_torord_step(row.ctypes.data, 0.0, DT, 0, 0, None)
+    return got, ref.T
+
+
+def _torord(state, values):
+    y = np.repeat(np.array(oracle.torord_initial_state(0))[:, None], len(values), axis=1)
+    y[state] = values
+    return y
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("state", [2, 4, 6, 9])
+def test_concentration_below_zero_is_reported(state, precision):
+    """A concentration whose logarithm, root or power does not exist makes V NaN, which the
+    loop reports (MB_ERR_NAN), and does not leave finite numbers behind: subspace Ca, Na and
+    K below the root of the ionic strength, myoplasmic Ca below zero."""
+    scale = 1.0 if state == 9 else 1000.0
+    y = _torord(state, -scale * np.array([1e-6, 3e-4, 0.5, 3.0]))
+    got, ref = _steps("torord", precision, y)
+    bad = np.isnan(ref[0])
+    assert bad.any()
+    assert np.array_equal(np.isnan(got[0]), bad)
