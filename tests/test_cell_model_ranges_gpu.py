@@ -57,3 +57,15 @@ def test_concentration_below_zero_is_reported(state, precision):
     bad = np.isnan(ref[0])
     assert bad.any()
     assert np.array_equal(np.isnan(got[0]), bad)
+
+
+@pytest.mark.parametrize("precision,low,high", [("fp64", -3000.0, 9000.0), ("mixed", -1400.0, 1100.0)])
+def test_potential_far_out(precision, low, high):
+    """ten Tusscher 2006 where the reference's formulas stay finite: m's time constant is a
+    product and a sum of reciprocals whose own reciprocals overflow much earlier."""
+    v = np.concatenate([np.linspace(low, high, 601), [399.5, 408.8, 430.0]])
+    y = np.repeat(np.array(oracle.tt2006_initial_state())[:, None], v.size, axis=1)
+    y[0] = v
+    got, ref = _steps("tt2006", precision, y)
+    assert np.isfinite(ref).all()
+    np.testing.assert_allclose(got, ref, rtol=1e-9 if precision == "fp64" else 1e-3, atol=1e-9)
