@@ -269,11 +269,12 @@ __device__ __forceinline__ void torord_step(IO &io, const T stim, const T dt, co
             const T g = PCa * d, pp = T(1.1) * p;
             oss = g * (q * (f * (T(1.0) - nca) + fca * nca) + pp * (fp * (T(1.0) - nca) + fcap * nca));
             oi = g * (q * (f * (T(1.0) - nca_i) + fca * nca_i) + pp * (fp * (T(1.0) - nca_i) + fcap * nca_i));
-            // n gate: anca = 1 / (k2n/km2n + (1 + Kmn/c)^4) with t = c / (c + Kmn), km2n = jca
-            const T k2n = T(500.0);
+            // n gate: anca = 1 / (k2n/km2n + (1 + Kmn/c)^4) with t = c / (c + Kmn), km2n = jca;
+            // 0 where jca and c are both 0 (tiny is below the last place of everything else)
+            const T k2n = T(500.0), tiny = T(1e-30);
             const T t4 = sq(sq(mdiv(cass, cass + T(0.002)))), u4 = sq(sq(mdiv(cai, cai + T(0.002))));
-            io.euler(32, nca, k2n * mdiv(t4 * jca, k2n * t4 + jca) - nca * jca);
-            io.euler(33, nca_i, k2n * mdiv(u4 * jca, k2n * u4 + jca) - nca_i * jca);
+            io.euler(32, nca, k2n * mdiv(t4 * jca, k2n * t4 + (jca + tiny)) - nca * jca);
+            io.euler(33, nca_i, k2n * mdiv(u4 * jca, k2n * u4 + (jca + tiny)) - nca_i * jca);
             T dss = T(1.0763) * mexp(T(-1.0070) * mexp(T(-0.0829) * v));
             if (v > T(31.4978)) dss = T(1);
             const T sd = mexp(T(-0.05) * (v + T(6.0))) + mexp(T(0.09) * (v + T(14.0)));
@@ -433,7 +434,9 @@ __device__ __forceinline__ void torord_step(IO &io, const T stim, const T dt, co
     {
         const T cansr = io.get(7), cajsr = io.get(8), Jnp = io.get(41), Jp = io.get(42);
         const T bt = T(4.75), btp = T(1.25) * T(4.75);
-        const T c8 = sq(sq(sq(cajsr))), r8 = sq(sq(sq(T(1.7))));
+        T c2 = sq(cajsr);
+        if constexpr (sizeof(T) == 4) c2 = c2 > T(1e8) ? T(1e8) : c2;   // c2^4 fits; the quotient is 1 from far below
+        const T c8 = sq(sq(c2)), r8 = sq(sq(sq(T(1.7))));
         T inf = T(0.5) * bt * (-ICaL) * mdiv(c8, c8 + r8);              // 1 / (1 + (1.7 / cajsr)^8)
         if (MID) inf = inf * T(1.7);
         const T r = mdiv(cajsr, cajsr + T(0.0123));

@@ -69,3 +69,15 @@ def test_potential_far_out(precision, low, high):
     got, ref = _steps("tt2006", precision, y)
     assert np.isfinite(ref).all()
     np.testing.assert_allclose(got, ref, rtol=1e-9 if precision == "fp64" else 1e-3, atol=1e-9)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_vanishing_and_large_quotients(precision):
+    """ToRORd states at which a quotient formed from products is 0/0 or overflows where the
+    reference's nested form has its limit: no calcium with jca = 0, a huge junctional SR load."""
+    y = _torord(8, [1e6, 1e5, 1.5, 1.5, 1.5, 1.5])
+    y[2, 2] = y[9, 3] = y[2, 4] = y[9, 5] = 0.0
+    y[29, 2] = y[29, 3] = 0.0
+    got, ref = _steps("torord", precision, y)
+    assert np.isfinite(ref).all()
+    np.testing.assert_allclose(got, ref, rtol=1e-9 if precision == "fp64" else 1e-3, atol=1e-7)
