@@ -120,7 +120,7 @@ struct mb_ode {
     int neq;
     double *d_stim;
     double *d_dense;       /* the state as neq rows of n, for get / set_state: made at the first
-                              call and kept up to MB_DENSE_KEPT bytes */
+                              call and kept up to MB_DENSE_KEPT bytes; NULL while a call uses it */
     cudaStream_t stream;
 };
 
@@ -235,31 +235,50 @@ int mb_solve_model_odes_gpu(mb_ode *o, double current_t, const double *stim_curr
 
 #define MB_DENSE_KEPT ((size_t)256 << 20)
 
-static void dense_done(mb_ode *o) {
-    if ((size_t)o->neq * o->dev.n * sizeof(double) <= MB_DENSE_KEPT) return;
-    cudaFree(o->d_dense);
-    o->d_dense = NULL;
+/* The object's dense buffer, or a new one while another thread's call has it. */
+static double *dense_take(mb_ode *o) {
+    double *d = __atomic_exchange_n(&o->d_dense, NULL, __ATOMIC_ACQ_REL);
+    if (!d && cudaMalloc((void **)&d, (size_t)o->neq * o->dev.n * sizeof(double)) != cudaSuccess) return NULL;
+    return d;
+}
+
+static void dense_put(mb_ode *o, double *d) {
+    double *none = NULL;
+    if ((size_t)o->neq * o->dev.n * sizeof(double) <= MB_DENSE_KEPT &&
+        __atomic_compare_exchange_n(&o->d_dense, &none, d, 0, __ATOMIC_ACQ_REL, __ATOMIC_RELAXED))
+        return;
+    cudaFree(d);
 }
 
 int mb_ode_get_state(mb_ode *o, double *host_state) {
     if (!o || !host_state) return set_err(MB_ERR_ARG, "null argument");
     const size_t bytes = (size_t)o->neq * o->dev.n * sizeof(double);
-    if (!o->d_dense) CK(cudaMalloc((void **)&o->d_dense, bytes));
-    CKK(mbk_ode_gather(&o->dev, NULL, o->d_dense, o->stream));
-    CK(cudaMemcpyAsync(host_state, o->d_dense, bytes, cudaMemcpyDeviceToHost, o->stream));
-    CK(cudaStreamSynchronize(o->stream));
-    dense_done(o);
+    double *d = dense_take(o);
+    if (!d) {
+        cudaGetLastError();
+        return set_err(MB_ERR_CUDA, "no device memory for %zu bytes of cell state", bytes);
+    }
+    cudaError_t e = (cudaError_t)mbk_ode_gather(&o->dev, NULL, d, o->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host_state, d, bytes, cudaMemcpyDeviceToHost, o->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(o->stream);
+    dense_put(o, d);
+    CK(e);
     return MB_OK;
 }
 
 int mb_ode_set_state(mb_ode *o, const double *host_state) {
     if (!o || !host_state) return set_err(MB_ERR_ARG, "null argument");
     const size_t bytes = (size_t)o->neq * o->dev.n * sizeof(double);
-    if (!o->d_dense) CK(cudaMalloc((void **)&o->d_dense, bytes));
-    CK(cudaMemcpyAsync(o->d_dense, host_state, bytes, cudaMemcpyHostToDevice, o->stream));
-    CKK(mbk_ode_scatter(&o->dev, o->d_dense, NULL, o->stream));
-    CK(cudaStreamSynchronize(o->stream));
-    dense_done(o);
+    double *d = dense_take(o);
+    if (!d) {
+        cudaGetLastError();
+        return set_err(MB_ERR_CUDA, "no device memory for %zu bytes of cell state", bytes);
+    }
+    cudaError_t e = cudaMemcpyAsync(d, host_state, bytes, cudaMemcpyHostToDevice, o->stream);
+    if (e == cudaSuccess) e = (cudaError_t)mbk_ode_scatter(&o->dev, d, NULL, o->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(o->stream);
+    dense_put(o, d);
+    CK(e);
     return MB_OK;
 }
 
