@@ -50,6 +50,13 @@ __device__ __forceinline__ bool grid_barrier(const Args &a, int &red) {
 }
 
 template <int LANES>
+__device__ __forceinline__ int row_max(int e) {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    return e;
+}
+
+template <int LANES>
 __device__ __forceinline__ double row_sum(double s) {
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -75,19 +82,20 @@ __global__ void __launch_bounds__(NT) k_csr_pcg(mb_csr_dev m, Args a) {
     // f(row, lane 0 of an existing row, the row's product with x).
     auto rows = [&](const double *x, bool diag, auto f) {
         for (int row = first_row; row - first_row % (32 / LANES) < m.n; row += per) {
-            double s = 0.0, d = 0.0;
+            double s = 0.0;
+            int at = -1;            // the row's diagonal entry (the last one, if it has several)
             if (row < m.n) {
                 const int e1 = m.row_ptr[row + 1];
                 for (int e = m.row_ptr[row] + lane; e < e1; e += LANES) {
                     const int col = m.col[e];
                     const double val = m.val[e];
                     s += val * __ldcg(x + col);
-                    if (diag && col == row) d = val;
+                    if (diag && col == row) at = e;
                 }
             }
             s = row_sum<LANES>(s);
-            if (diag) d = row_sum<LANES>(d);
-            if (lane == 0 && row < m.n) f(row, s, d);
+            if (diag) at = row_max<LANES>(at);
+            if (lane == 0 && row < m.n) f(row, s, at >= 0 ? m.val[at] : 0.0);
         }
     };
     zero();

@@ -54,3 +54,51 @@ def test_matches_oracle(n, band, pre):
         np.testing.assert_allclose(x, xr, rtol=0, atol=1e-10 * max(1.0, np.abs(xr).max()))
     again, i, _ = csr_conjugate_gradient(ptr, col, val, b, xr, 1.0 + er, 200, pre)
     assert i == 1 and np.array_equal(again, xr)          # already below the tolerance: nothing moves
+
+
+def _pcg(ptr, col, val, b, inv, tol):
+    """Jacobi-PCG with the given 1/diag (its, x), the iteration of cpu_conjugate_gradient."""
+    rows = np.repeat(np.arange(b.size), np.diff(ptr))
+    mul = lambda p: np.bincount(rows, val * p[col], b.size)  # noqa: E731
+    x, r = np.zeros_like(b), b.copy()
+    p = inv * r
+    rz, its = r @ p, 1
+    while r @ r >= tol and its < 200:
+        q = mul(p)
+        alpha = rz / (p @ q)
+        x += alpha * p
+        r -= alpha * q
+        z = inv * r
+        rz, old = r @ z, rz
+        p = z + rz / old * p
+        its += 1
+        if r @ r <= tol:
+            break
+    return its, x
+
+
+@pytest.mark.parametrize("n,band", [(700, 2), (600, 20)])
+def test_repeated_diagonal_entries(n, band):
+    """A row whose diagonal comes in several entries is preconditioned by the last of
+    them, wherever in the row they lie (the product takes their sum)."""
+    from monoalg3d_c_b200 import csr_conjugate_gradient
+    ptr, col, val = _spd(n, band, 5)
+    rng = np.random.default_rng(6)
+    out, cols, vals, inv = [0], [], [], np.empty(n)
+    for i in range(n):
+        c, v = list(col[ptr[i] + 1:ptr[i + 1]]), list(val[ptr[i] + 1:ptr[i + 1]])
+        parts = val[ptr[i]] * rng.dirichlet(np.full(3, 4.0))
+        at = sorted(rng.integers(0, len(c) + 1, 3), reverse=True)
+        for k, d in zip(at, parts):
+            c.insert(k, i)
+            v.insert(k, d)
+        cols += c
+        vals += v
+        inv[i] = 1.0 / v[len(c) - 1 - c[::-1].index(i)]
+        out.append(len(cols))
+    ptr, col, val = np.array(out, dtype=np.int32), np.array(cols, dtype=np.int32), np.array(vals)
+    b = rng.standard_normal(n)
+    its, x = _pcg(ptr, col, val, b, inv, 1e-20)
+    got, i, _ = csr_conjugate_gradient(ptr, col, val, b, None, 1e-20, 200, True)
+    assert 10 < its < 200 and abs(i - its) <= 1
+    np.testing.assert_allclose(got, x, rtol=0, atol=1e-9 * np.abs(x).max())
