@@ -178,9 +178,10 @@ __global__ void __launch_bounds__(NT) k_csr_pcg(mb_csr_dev m, Args a) {
 
 using namespace mb::csr;
 
+// Lanes per row: its entries in a few sectors each.
+static int lanes_of(int32_t n, int32_t nnz) { return nnz / n <= 16 ? 4 : 16; }
 static const void *kernel_of(int32_t n, int32_t nnz) {
-    // lanes per row: its entries in a few sectors each
-    return nnz / n <= 16 ? (const void *)k_csr_pcg<4> : (const void *)k_csr_pcg<16>;
+    return lanes_of(n, nnz) == 4 ? (const void *)k_csr_pcg<4> : (const void *)k_csr_pcg<16>;
 }
 
 // Blocks of the cooperative launch: all that fit at once, no more than the rows
@@ -190,7 +191,7 @@ extern "C" int mbk_csr_pcg_blocks(int32_t n, int32_t nnz) {
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel_of(n, nnz), NT, 0) != cudaSuccess || per < 1) return -1;
-    const long long want = ((long long)n * 4 + NT - 1) / NT;
+    const long long want = ((long long)n * lanes_of(n, nnz) + NT - 1) / NT;
     const int most = sms * (per > 2 ? 2 : per);
     return want < most ? (int)want : most;
 }

@@ -102,3 +102,11 @@ def test_repeated_diagonal_entries(n, band):
     got, i, _ = csr_conjugate_gradient(ptr, col, val, b, None, 1e-20, 200, True)
     assert 10 < its < 200 and abs(i - its) <= 1
     np.testing.assert_allclose(got, x, rtol=0, atol=1e-9 * np.abs(x).max())
+
+
+@pytest.mark.parametrize("n,nnz,blocks", [(1, 1, 1), (128, 16 * 128, 1), (129, 16 * 129, 2), (900, 40 * 900, 29),
+                                          (33, 17 * 33, 2)])
+def test_blocks_cover_the_rows(n, nnz, blocks):
+    """A small solve gets a block for every 512 lanes its rows take (4 or 16 lanes a row)."""
+    from monoalg3d_c_b200._lib import lib
+    assert lib.mbk_csr_pcg_blocks(n, nnz) == blocks
