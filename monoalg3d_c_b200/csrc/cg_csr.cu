@@ -2,14 +2,20 @@
 // (mb_csr_solve): the iteration and stopping rule of cpu_conjugate_gradient
 // (linear_system_solver.c:47-183), one reduction and one barrier per iteration.
 //
-// Why: with a kernel per phase an iteration was three launches with their
-// gaps, 24 us of kernels on a 200 k-row 7-point matrix whose 17 MB stay in L2, and the
-// host read the stopping flag back every 16 iterations.
+// Why: with a kernel per phase (cg_kernels.cu:k_csr_*) an iteration is three launches
+// with their gaps, and the host reads the stopping flag back every 16 iterations: 30 us
+// an iteration on a 200 k-row 7-point matrix whose 17 MB stay in L2, 16 us here.
 //
 // A part of a warp (LANES lanes) takes a row, so that its entries are read
-// as whole sectors.  Per iteration: x, r and p of the rows, a grid barrier (p of
+// as whole sectors, R rows at a time: bound by the latency of row pointer, entry and
+// vector value, one after the other.  R = 4 fits 64 registers, two blocks per SM; with one
+// row at a time the kernel took 126, one block (22 us), R = 2 took 18 us and R = 8, 106
+// registers, 17 us.  Once matrix and vectors leave L2 this is not enough: the phases'
+// thread per row keeps four times the rows in flight (mbk_csr_in_l2).
+// Per iteration: x, r and p of the rows, a grid barrier (p of
 // other rows is read next), then q = A p and the sums p.q, q.z, q.Mq, q.r, q.q,
 // r.z, r.r for the next r.z and r.r (cg_cluster.cu, with its guard).
+#include <type_traits>
 #include "cg_common.cuh"
 
 namespace mb {
@@ -20,6 +26,7 @@ using fcg::grid_reduce8;
 using fcg::SPIN_LIMIT;
 
 constexpr int NT = 512;
+constexpr int R = 4;
 constexpr double GUARD = 1e-4;
 
 // Grid-wide barrier on the reductions' arrival counter.
@@ -78,28 +85,57 @@ __global__ void __launch_bounds__(NT) k_csr_pcg(mb_csr_dev m, Args a) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = 0.0;
     };
-    // Every warp runs the same number of rounds (the row sums' shuffles):
-    // f(row, lane 0 of an existing row, the row's product with x).
-    auto rows = [&](const double *x, bool diag, auto f) {
-        for (int row = first_row; row - first_row % (32 / LANES) < m.n; row += per) {
-            double s = 0.0;
-            int at = -1;            // the row's diagonal entry (the last one, if it has several)
-            if (row < m.n) {
-                const int e1 = m.row_ptr[row + 1];
-                for (int e = m.row_ptr[row] + lane; e < e1; e += LANES) {
-                    const int col = m.col[e];
-                    const double val = m.val[e];
-                    s += val * __ldcg(x + col);
-                    if (diag && col == row) at = e;
+    // f(row, lane 0 of an existing row, the row's product with x).  R rows of a thread
+    // at once, so that their entries are in flight together; every warp runs the same
+    // number of rounds (the row sums' shuffles).
+    auto rows = [&](const double *x, auto with_diag, auto f) {
+        constexpr bool diag = decltype(with_diag)::value;
+        for (int row0 = first_row; row0 - first_row % (32 / LANES) < m.n; row0 += R * per) {
+            int e[R], e1[R], at[R];     // at: the row's diagonal entry (the last one, if it has several)
+            double s[R];
+            bool more = false;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int row = row0 + k * per;
+                const bool in = row < m.n;
+                e[k] = in ? m.row_ptr[row] + lane : 0;
+                e1[k] = in ? m.row_ptr[row + 1] : 0;
+                s[k] = 0.0;
+                at[k] = -1;
+            }
+#pragma unroll
+            for (int k = 0; k < R; ++k) more |= e[k] < e1[k];
+            while (more) {
+                int col[R];
+                double val[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    const bool in = e[k] < e1[k];
+                    col[k] = in ? m.col[e[k]] : 0;
+                    val[k] = in ? m.val[e[k]] : 0.0;
+                }
+                more = false;
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    if (e[k] < e1[k]) {
+                        s[k] += val[k] * __ldcg(x + col[k]);
+                        if (diag && col[k] == row0 + k * per) at[k] = e[k];
+                    }
+                    e[k] += LANES;
+                    more |= e[k] < e1[k];
                 }
             }
-            s = row_sum<LANES>(s);
-            if (diag) at = row_max<LANES>(at);
-            if (lane == 0 && row < m.n) f(row, s, at >= 0 ? m.val[at] : 0.0);
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int row = row0 + k * per;
+                const double sum = row_sum<LANES>(s[k]);
+                const int d = diag ? row_max<LANES>(at[k]) : -1;
+                if (lane == 0 && row < m.n) f(row, sum, d >= 0 ? m.val[d] : 0.0);
+            }
         }
     };
     zero();
-    rows(m.x, true, [&](int row, double ax, double d) {
+    rows(m.x, std::true_type{}, [&](int row, double ax, double d) {
         const double id = 1.0 / (d == 0.0 ? 1.0 : d), r = m.b[row] - ax, z = pre ? id * r : r;
         m.inv_diag[row] = id;
         m.r[row] = r;
@@ -128,7 +164,7 @@ __global__ void __launch_bounds__(NT) k_csr_pcg(mb_csr_dev m, Args a) {
             if (!grid_barrier(a, red)) return;
         }
         zero();
-        rows(m.p, false, [&](int row, double q, double) {
+        rows(m.p, std::false_type{}, [&](int row, double q, double) {
             const double r = __ldcg(m.r + row), id = pre ? __ldcg(m.inv_diag + row) : 1.0, z = id * r;
             m.q[row] = q;
             v[0] += __ldcg(m.p + row) * q;
@@ -194,6 +230,15 @@ extern "C" int mbk_csr_pcg_blocks(int32_t n, int32_t nnz) {
     const long long want = ((long long)n * lanes_of(n, nnz) + NT - 1) / NT;
     const int most = sms * (per > 2 ? 2 : per);
     return want < most ? (int)want : most;
+}
+
+// Whether the one-launch solve is the faster: while the matrix (12 B an entry) and the
+// vectors (56 B a row) stay in L2.  Measured per iteration, here and by phases: 600 k rows
+// of 7 entries (84 MB) 34 and 43 us, 50 k rows of 152 (94 MB) 37 and 58 us, but 200 k
+// rows of 38 (105 MB) 60 and 56 us, 900 k rows of 7 (125 MB) 76 and 64 us, 2 M rows 186 and
+// 116 us.
+extern "C" int mbk_csr_in_l2(int32_t n, int32_t nnz) {
+    return 12LL * nnz + 56LL * n <= (96LL << 20);
 }
 
 // bar: 2 words; partials: 16 values per block.

@@ -187,6 +187,7 @@ int mbk_csr_cg_iter(const mb_csr_dev *a, mb_ctrl *ctrl, cudaStream_t s);
 
 /* the whole solve in one cooperative launch (cg_csr.cu); partials: 16 values per block */
 int mbk_csr_pcg_blocks(int32_t n, int32_t nnz);
+int mbk_csr_in_l2(int32_t n, int32_t nnz);
 int mbk_csr_pcg(const mb_csr_dev *a, int32_t nnz, int blocks, mb_ctrl *ctrl, double *partials, unsigned *bar, int *status,
                 cudaStream_t s);
 

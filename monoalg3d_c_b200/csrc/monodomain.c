@@ -1743,7 +1743,7 @@ struct mb_csr {
     mb_ctrl *d_ctrl;
     unsigned *d_bar;       /* 2 words of the grid barrier, then the status word */
     int32_t nnz;
-    int blocks;            /* of the cooperative solve */
+    int blocks;            /* of the cooperative solve, 0: a kernel per phase */
     cudaStream_t s;
 };
 
@@ -1764,10 +1764,14 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     mb_csr *m = (mb_csr *)calloc(1, sizeof *m);
     if (!m) return set_err(MB_ERR_NOMEM, "out of host memory");
     m->nnz = nnz;
-    m->blocks = mbk_csr_pcg_blocks(n, nnz);
-    if (m->blocks < 1) {
-        free(m);
-        return set_err(MB_ERR_CUDA, "mb_csr_create: no device for the cooperative solve");
+    int gb = (n + 255) / 256;
+    if (gb > mbk_max_grid_blocks()) gb = mbk_max_grid_blocks();
+    if (mbk_csr_in_l2(n, nnz)) {
+        m->blocks = mbk_csr_pcg_blocks(n, nnz);
+        if (m->blocks < 1) {
+            free(m);
+            return set_err(MB_ERR_CUDA, "mb_csr_create: no device for the cooperative solve");
+        }
     }
     cudaError_t e = cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking);
 #define CSR_ALLOC(p, bytes) if (e == cudaSuccess) e = cudaMalloc((void **)&(p), (bytes))
@@ -1780,7 +1784,7 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     CSR_ALLOC(m->d_p, (size_t)n * sizeof(double));
     CSR_ALLOC(m->d_q, (size_t)n * sizeof(double));
     CSR_ALLOC(m->d_id, (size_t)n * sizeof(double));
-    CSR_ALLOC(m->d_part, (size_t)16 * m->blocks * sizeof(double));
+    CSR_ALLOC(m->d_part, (size_t)(m->blocks ? 16 * m->blocks : 3 * gb) * sizeof(double));
     CSR_ALLOC(m->d_ctrl, sizeof(mb_ctrl));
     CSR_ALLOC(m->d_bar, 3 * sizeof(unsigned));
 #undef CSR_ALLOC
@@ -1793,7 +1797,7 @@ int mb_csr_create(mb_csr **out, int32_t n, const int32_t *row_ptr, const int32_t
     }
     mb_csr_dev *a = &m->a;
     a->n = n;
-    a->grid_blocks = m->blocks;
+    a->grid_blocks = gb;
     a->row_ptr = m->d_rp; a->col = m->d_col; a->val = m->d_val; a->b = m->d_b; a->x = m->d_x;
     a->r = m->d_r; a->p = m->d_p; a->q = m->d_q; a->inv_diag = m->d_id; a->partials = m->d_part;
     *out = m;
@@ -1813,7 +1817,17 @@ int mb_csr_solve(mb_csr *m, const double *b, double *x, double tolerance, int ma
     c.use_precond = use_preconditioner ? 1 : 0;
     CK(cudaMemcpyAsync(m->d_ctrl, &c, sizeof c, cudaMemcpyHostToDevice, m->s));
     CK(cudaMemsetAsync(m->d_bar + 2, 0, sizeof(unsigned), m->s));
-    CKK(mbk_csr_pcg(&m->a, m->nnz, m->blocks, m->d_ctrl, m->d_part, m->d_bar, (int *)(m->d_bar + 2), m->s));
+    if (m->blocks)
+        CKK(mbk_csr_pcg(&m->a, m->nnz, m->blocks, m->d_ctrl, m->d_part, m->d_bar, (int *)(m->d_bar + 2), m->s));
+    else
+        CKK(mbk_csr_cg_init(&m->a, m->d_ctrl, m->s));
+    for (int it = 0; !m->blocks && it < max_iterations + 1; it += 16) {
+        for (int q = 0; q < 16; ++q) CKK(mbk_csr_cg_iter(&m->a, m->d_ctrl, m->s));
+        int32_t done = 0;
+        CK(cudaMemcpyAsync(&done, &m->d_ctrl->done, sizeof done, cudaMemcpyDeviceToHost, m->s));
+        CK(cudaStreamSynchronize(m->s));
+        if (done) break;
+    }
     unsigned status = 0;
     CK(cudaMemcpyAsync(&c, m->d_ctrl, sizeof c, cudaMemcpyDeviceToHost, m->s));
     CK(cudaMemcpyAsync(&status, m->d_bar + 2, sizeof status, cudaMemcpyDeviceToHost, m->s));

@@ -110,3 +110,25 @@ def test_blocks_cover_the_rows(n, nnz, blocks):
     """A small solve gets a block for every 512 lanes its rows take (4 or 16 lanes a row)."""
     from monoalg3d_c_b200._lib import lib
     assert lib.mbk_csr_pcg_blocks(n, nnz) == blocks
+
+
+@pytest.mark.parametrize("n", [870_000, 1_400_003])
+def test_beyond_l2(n):
+    """Matrices that stay in L2 are solved in one launch, larger ones by a kernel per
+    phase, with the same iterations: a chain of n rows on either side of the line
+    (matrix and vectors 80 and 128 MB)."""
+    from monoalg3d_c_b200 import csr_conjugate_gradient
+    from monoalg3d_c_b200._lib import lib
+    i = np.arange(n)
+    col = np.stack([i, (i - 1) % n, (i + 1) % n], axis=1).reshape(-1)
+    val = np.tile([2.5, -1.0, -1.0], n)
+    val[1] = val[-1] = 0.0                     # no wrap-around
+    ptr = np.arange(n + 1) * 3
+    assert lib.mbk_csr_in_l2(n, 3 * n) == (n < 1_000_000)
+    rng = np.random.default_rng(4)
+    b = rng.standard_normal(n)
+    for most in (200, 17):
+        xr, ir, er = oracle.pcg(ptr.astype(np.int32), col.astype(np.int32), val, b, np.zeros(n), 1e-8, most, True)
+        x, k, e = csr_conjugate_gradient(ptr, col, val, b, None, 1e-8, most, True)
+        assert k == ir and e == pytest.approx(er, rel=1e-6)
+        np.testing.assert_allclose(x, xr, rtol=0, atol=1e-10 * np.abs(xr).max())
