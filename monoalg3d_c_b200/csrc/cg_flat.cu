@@ -31,8 +31,8 @@
 // iteration restarts from it; the stopping test uses that FP64 residual.
 //
 // Launch shapes are template parameters (threads per block, cells gathered
-// per thread before use, resident blocks per SM); the host times the
-// variants on the tissue's first solve and keeps the fastest.
+// per thread before use, resident blocks per SM); the host times a few of them
+// (monodomain.c:cg_autotune) when the tissue is made and keeps the fastest.
 #include "cg_rows.cuh"
 #include "mb_math.cuh"
 
@@ -915,19 +915,25 @@ struct Variant {
 // four-cell groups); the group variants need nx to be a multiple of 4
 #define MB_SHAPES(K, O)                                                                                          \
     {(const void *)k_fcg<MIXED, K, 1024, 1, 1, false, O>, 1024, 0, 1},                                      \
+        {(const void *)k_fcg<MIXED, K, 1024, 1, 2, false, O>, 1024, 0, 1},                                  \
         {(const void *)k_fcg<MIXED, K, 512, 2, 2, false, O>, 512, 0, 2},                                    \
+        {(const void *)k_fcg<MIXED, K, 512, 1, 4, false, O>, 512, 0, 1},                                    \
+        {(const void *)k_fcg<MIXED, K, 256, 2, 4, false, O>, 256, 0, 2},                                    \
         {(const void *)k_fcg<MIXED, K, 1024, 1, 1, true, O>, 1024, 1, 1},                                   \
         {(const void *)k_fcg<MIXED, K, 512, 1, 2, true, O>, 512, 1, 1},                                     \
+        {(const void *)k_fcg<MIXED, K, 256, 1, 4, true, O>, 256, 1, 1},                                     \
         {(const void *)k_fcg<MIXED, K, 512, 2, 1, true, O>, 512, 1, 2},                                     \
         {(const void *)k_fcg<MIXED, K, 256, 2, 2, true, O>, 256, 1, 2},                                     \
         {(const void *)k_fcg<MIXED, K, 512, 1, 1, true, O>, 512, 1, 1},                                     \
         {(const void *)k_fcg<MIXED, K, 256, 1, 2, true, O>, 256, 1, 1}
-// variants 0..7: each block sweeps its own range; 8..15: the same shapes
+// variants 0..11: each block sweeps its own range; 12..23: the same shapes
 // with the interleaved sweep.  The last two shapes give a thread 128
-// registers, enough for every row load of a 27-point group in flight.
+// registers, enough for every row load of a 27-point group in flight.  The numbers
+// are what MB_CG_VARIANT takes: a shape the tuner no longer times keeps its own, so
+// that a run that names one gives the same bits.
 #define MB_VARIANTS(K) MB_SHAPES(K, 0), MB_SHAPES(K, 1)
 
-constexpr int NUM_VARIANTS = 16;
+constexpr int NUM_VARIANTS = 24;
 
 template <bool MIXED>
 static Variant variant_of(int kind, int v) {
