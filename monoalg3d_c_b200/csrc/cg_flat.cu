@@ -32,7 +32,7 @@
 //
 // Launch shapes are template parameters (threads per block, cells gathered
 // per thread before use, resident blocks per SM); the host times a few of them
-// (monodomain.c:cg_autotune) when the tissue is made and keeps the fastest.
+// (monodomain.c:cg_candidates) when the tissue is made and keeps the fastest.
 #include "cg_rows.cuh"
 #include "mb_math.cuh"
 

@@ -56,7 +56,6 @@ struct mb_monodomain {
     double *d_apb;               /* the same in FP64 (flat fused form) */
     unsigned *d_bar;
     int *d_status;
-    float cg_tune_ms;     /* device time of one CG solve of the chosen kernel at tuning */
 
     mb_ode_dev ode;
     mb_stencil_dev st;

@@ -472,41 +472,116 @@ static int pcg_launch(const mb_pcg_dev *q, cudaStream_t s) {
     }
 }
 
-/* Picks the CG kernel: every launch-shape variant of the flat persistent
- * kernel, the 2.5D tiled one, where its tiles fit the resident one, for
- * the 27-point class-table operator every variant of the z-march kernel,
- * where the vectors fit a cluster's shared memory every cluster size of the
- * cluster kernel, and the fused flat form's shapes solve one system; V is restored after every trial and the
- * fastest by CUDA events is kept.  The system is the tissue's first one with up to
- * 5 mV of noise on V*, so that it takes as many iterations as a step with
+/* The CG kernels by number (MB_CG_VARIANT): the flat shapes, the 2.5D tiled kernel, the
+ * resident one, the z-march variants, the clusters of 2^v blocks, the fused flat
+ * shapes. */
+enum { CG_TILED, CG_RESIDENT, CG_ZMARCH, CG_CLUSTER, CG_FUSED, CG_END };
+static int cg_number(int group) {
+    const int nv = mbk_fcg_variants(0), z0 = nv + 2, c0 = z0 + mbk_zcg_variants(), f0 = c0 + mbk_ccg_variants();
+    const int at[] = {nv, nv + 1, z0, c0, f0, f0 + mbk_ffcg_variants()};
+    return at[group];
+}
+
+/* Makes q the launch of kernel number cand; 0 where it does not run on this tissue. */
+static int cg_select(const mb_monodomain *m, int cand, mb_pcg_dev *q) {
+    const int mixed = m->desc.precision == MB_PREC_MIXED, kind = m->st.kind, whole = m->desc.nx % 4 == 0;
+    if (cand < 0 || cand >= cg_number(CG_END)) return 0;
+    if (cand >= cg_number(CG_FUSED)) {
+        q->form = MB_PCG_FUSED;
+        q->variant = cand - cg_number(CG_FUSED);
+        if (!mbk_ffcg_usable(&m->st) || (mbk_ffcg_variant_groups(q->variant) && !whole)) return 0;
+        q->blocks = mbk_ffcg_max_blocks(mixed, kind, q->variant);
+    } else if (cand >= cg_number(CG_CLUSTER)) {
+        q->form = MB_PCG_CLUSTER;
+        q->cc_variant = cand - cg_number(CG_CLUSTER);
+        if (!mbk_ccg_usable(q, q->cc_variant)) return 0;
+        q->blocks = 1 << q->cc_variant;
+    } else if (cand >= cg_number(CG_ZMARCH)) {
+        q->form = MB_PCG_ZMARCH;
+        q->zc_variant = cand - cg_number(CG_ZMARCH);
+        if (!mbk_zcg_variant_usable(&m->st, mixed, q->zc_variant)) return 0;
+        q->blocks = mbk_zcg_max_blocks(mixed, q->zc_variant);
+    } else if (cand == cg_number(CG_RESIDENT)) {
+        if (!mbk_rcg_plan(q)) return 0;
+        q->form = MB_PCG_RESIDENT;
+        q->blocks = q->rc_nbx * q->rc_nby;
+    } else if (cand == cg_number(CG_TILED)) {
+        const int most = mbk_tcg_max_blocks(mixed);
+        mbk_tcg_layout(m->desc.nx, m->desc.ny, m->desc.nz, most > 0 ? most : 1, &q->tiles_x, &q->tiles_y, &q->zchunk,
+                       &q->nchunks);
+        q->form = MB_PCG_TILED;
+        const int items = q->tiles_x * q->tiles_y * q->nchunks;
+        q->blocks = items < most ? items : most;
+    } else {
+        q->form = MB_PCG_FLAT;
+        q->variant = cand;
+        if (mbk_fcg_variant_groups(cand) && !whole) return 0;
+        q->blocks = mbk_fcg_max_blocks(mixed, kind, cand);
+    }
+    return q->blocks > 0;
+}
+
+/* The kernels that are timed for a tissue (at most CG_MAX_CANDIDATES numbers), those
+ * first that mostly win.  Creating a small tissue costs as much as hundreds of its
+ * steps, so the rule leaves out what is never the fastest, or by 2 % at most; measured on
+ * 56 tissues from 30 to 25 M cells in both precisions (us per solve, FP64 / mixed):
+ *   7-point, to 32 k cells: the cluster of 340 to 680 cells a block and the next larger
+ *     (400 cells 34 / 37, fused 51 / 69; 4096 cells 47 / 48, fused 72 / 87; 16 k cells
+ *     72, fused 76); at 65 k cells a cluster takes 111 / 114, the fused form 82 / 95;
+ *   7-point, to 2^20 cells: fused shape 0 and, with whole groups of 4 cells in a row,
+ *     shape 2, where a flat shape comes last to 2^18 cells (200 k 132 / 132, flat
+ *     144 / 137; 262 k 142 / 138, flat 158 / 147) and first from then on (400 k 199 / 217,
+ *     flat 225 / 201; 983 k 339 / 262, flat 342 / 246);
+ *   beyond: the flat shapes, with whole groups those of 4 cells a thread (2 M 602 / 366,
+ *     25 M 7500 / 4480), for a plane in FP64 one cell a thread (1 M 250, groups 291),
+ *     else one cell a thread (2 M 613 / 419);
+ *   27-point: the z-march variants and flat shape 12 (19 k cells 176 / 179, flat 176 / 186;
+ *     2 M 939 / 632, flat 1031 / 669; 25 M 8620 / 4530, flat 11400 / 7400), ragged rows
+ *     shape 0 too (500 k 470 / 366, flat 383 / 391); clusters to 8 k cells (4000 cells
+ *     162, z-march 172 / 178).
+ * The tiled and the resident kernel win nowhere any more; they run by number. */
+enum { CG_MAX_CANDIDATES = 12 };
+static int cg_candidates(const mb_monodomain *m, int *list) {
+    const int z0 = cg_number(CG_ZMARCH), c0 = cg_number(CG_CLUSTER), f0 = cg_number(CG_FUSED);
+    const int mixed = m->desc.precision == MB_PREC_MIXED, wide = m->st.kind == 2, whole = m->desc.nx % 4 == 0;
+    int n = 0;
+    const char *env = getenv("MB_CG_VARIANT");
+    if (env) {
+        list[n++] = atoi(env);
+        return n;
+    }
+    if (m->n <= (wide ? 8192 : 32768)) {
+        int v = 0;
+        while (v < mbk_ccg_variants() - 1 && m->n >= (680LL << v)) ++v;
+        list[n++] = c0 + v;
+        if (v + 1 < mbk_ccg_variants()) list[n++] = c0 + v + 1;
+    }
+    if (wide && mbk_zcg_usable(&m->st)) {
+        static const int z64[] = {0, 2, 5}, z32[] = {7, 8, 9, 0, 1};
+        for (int k = 0; k < (mixed ? 5 : 3); ++k) list[n++] = z0 + (mixed ? z32[k] : z64[k]);
+        list[n++] = 12;
+        if (!whole) list[n++] = 0;
+    } else {
+        static const int vec[] = {22, 10, 17, 8, 20, 0}, one[] = {12, 14, 0, 2};
+        const int few = mbk_ffcg_usable(&m->st) && m->n <= (1 << 18);
+        if (mbk_ffcg_usable(&m->st)) {
+            list[n++] = f0;
+            if (whole) list[n++] = f0 + 2;
+        }
+        for (int k = 0; k < (few ? 1 : whole ? 6 : 4); ++k) list[n++] = whole ? vec[k] : one[k];
+    }
+    return n;
+}
+
+/* Picks the CG kernel: the candidates solve one system; V is restored after every trial
+ * and the fastest by CUDA events is kept.  The system is the tissue's first one with up
+ * to 5 mV of noise on V*, so that it takes as many iterations as a step with
  * wave fronts does (the initial state alone is solved in one or two, which ranks
  * the kernels by their set-up).  A candidate's first run is not timed (it may load
- * the kernel); one whose second takes over 1.2 times the best is not run again.  MB_CG_VARIANT=<n> forces a choice (n = number of
- * flat variants selects the tiled kernel, n + 1 the resident kernel, n + 2 + v
- * z-march variant v, then the cluster of 2^v blocks, then fused shape v). */
-static int cg_autotune(mb_monodomain *m) {
+ * the kernel); one whose second takes over 1.2 times the best is not run again.
+ * MB_CG_VARIANT=<n> leaves kernel n alone (flat shape 0 where it does not run). */
+static int cg_autotune(mb_monodomain *m, const int *list, int count) {
     if (!m->use_pcg) return MB_OK;
-    const int mixed = m->pcg.mixed;
-    const int kind = m->st.kind;
-    const int nv = mbk_fcg_variants(kind);
-    int resident = mbk_rcg_plan(&m->pcg);
-    if (resident && !m->d_rtrue) {
-        if (cudaMalloc((void **)&m->d_rtrue, (size_t)m->n * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            m->d_rtrue = NULL;
-            resident = 0;
-        }
-        m->pcg.rtrue = m->d_rtrue;
-    }
-    const int zmarch = mbk_zcg_usable(&m->st) && m->pcg.zc_maps != NULL;
-    const int nzv = mbk_zcg_variants();
-    const char *env = getenv("MB_CG_VARIANT");
-    const int ncv = mbk_ccg_variants(), nfv = mbk_ffcg_variants();
-    /* candidates 0..nv-1 flat, nv tiled, nv+1 resident, nv+2.. z-march, then
-     * clusters, then the fused flat form */
-    const int c0 = nv + 2 + nzv, f0 = c0 + ncv;
-    int lo = 0, hi = f0 + nfv - 1;
-    if (env) lo = hi = atoi(env);
     double *vsave = NULL, *rhs = NULL;
     if (cudaMalloc((void **)&vsave, (size_t)m->n * sizeof(double)) != cudaSuccess)
         return set_err(MB_ERR_NOMEM, "CG tuning buffer");
@@ -519,53 +594,31 @@ static int cg_autotune(mb_monodomain *m) {
     }
     cudaMemcpyAsync(vsave, m->d_v, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
     float best = 1e30f;
-    int bestc = 0, rc = MB_OK;      /* variant 0 runs on every grid */
-    /* the specialised kernels first: where one applies it is the faster, and the
-     * others then end after their second run */
-    for (int cand = hi; cand >= lo && !rc; --cand) {
+    int rc = MB_OK;
+    mb_pcg_dev win = m->pcg;        /* flat shape 0 runs on every grid */
+    cg_select(m, 0, &win);
+    for (int k = 0; k < count && !rc; ++k) {
         mb_pcg_dev q = m->pcg;
-        if (rhs) q.vstar = rhs;
-        if (cand < nv) {
-            q.form = MB_PCG_FLAT;
-            q.variant = cand;
-            q.blocks = mbk_fcg_max_blocks(mixed, kind, cand);
-        } else if (cand == nv) {
-            q.form = MB_PCG_TILED;
-            const int items = q.tiles_x * q.tiles_y * q.nchunks;
-            const int mb = mbk_tcg_max_blocks(mixed);
-            q.blocks = items < mb ? items : mb;
-        } else if (cand == nv + 1) {
-            if (!resident) continue;
-            q.form = MB_PCG_RESIDENT;
-            q.blocks = q.rc_nbx * q.rc_nby;
-        } else if (cand >= f0) {
-            if (cand >= f0 + nfv || !mbk_ffcg_usable(&m->st)) continue;
-            q.form = MB_PCG_FUSED;
-            q.variant = cand - f0;
-            if (mbk_ffcg_variant_groups(q.variant) && (m->desc.nx % 4) != 0) continue;
-            q.blocks = mbk_ffcg_max_blocks(mixed, kind, q.variant);
-        } else if (cand >= c0) {
-            q.form = MB_PCG_CLUSTER;
-            q.cc_variant = cand - c0;
-            if (!mbk_ccg_usable(&q, q.cc_variant)) continue;
-            q.blocks = 1 << q.cc_variant;
-        } else {
-            if (!zmarch || !mbk_zcg_variant_usable(&m->st, mixed, cand - nv - 2)) continue;
-            q.form = MB_PCG_ZMARCH;
-            q.zc_variant = cand - nv - 2;
-            q.blocks = mbk_zcg_max_blocks(mixed, q.zc_variant);
+        if (!cg_select(m, list[k], &q)) continue;
+        if (q.form == MB_PCG_RESIDENT && !q.rtrue) {
+            if (cudaMalloc((void **)&m->d_rtrue, (size_t)m->n * sizeof(double)) != cudaSuccess) {
+                cudaGetLastError();
+                m->d_rtrue = NULL;
+                continue;
+            }
+            q.rtrue = m->d_rtrue;
         }
-        if (q.blocks <= 0) continue;
-        if (cand < nv && mbk_fcg_variant_groups(cand) && (m->desc.nx % 4) != 0) continue;
+        mb_pcg_dev run = q;
+        if (rhs) run.vstar = rhs;
         float tsum = 0;
         for (int rep = 0; rep < 3 && !rc; ++rep) {
             cudaMemcpyAsync(m->d_v, vsave, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
             forget_stored_product(m);
             cudaEventRecord(m->ev[0], m->stream);
-            const int e = pcg_launch(&q, m->stream);
+            const int e = pcg_launch(&run, m->stream);
             cudaEventRecord(m->ev[1], m->stream);
             if (e || cudaEventSynchronize(m->ev[1]) != cudaSuccess) {
-                rc = set_err(MB_ERR_CUDA, "CG tuning launch failed (candidate %d): %s", cand,
+                rc = set_err(MB_ERR_CUDA, "CG tuning launch failed (candidate %d): %s", list[k],
                              cudaGetErrorString(e ? (cudaError_t)e : cudaGetLastError()));
                 break;
             }
@@ -576,7 +629,7 @@ static int cg_autotune(mb_monodomain *m) {
         }
         if (!rc && tsum < best) {
             best = tsum;
-            bestc = cand;
+            win = q;
         }
     }
     cudaMemcpyAsync(m->d_v, vsave, (size_t)m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
@@ -588,31 +641,7 @@ static int cg_autotune(mb_monodomain *m) {
     int st = 0;
     cudaMemcpy(&st, m->d_status, sizeof st, cudaMemcpyDeviceToHost);
     if (st) return set_err(MB_ERR_CUDA, "CG grid barrier timed out during tuning");
-    if (bestc < nv) {
-        m->pcg.form = MB_PCG_FLAT;
-        m->pcg.variant = bestc;
-        m->pcg.blocks = mbk_fcg_max_blocks(mixed, kind, bestc);
-    } else if (bestc == nv) {
-        m->pcg.form = MB_PCG_TILED;
-        const int items = m->pcg.tiles_x * m->pcg.tiles_y * m->pcg.nchunks;
-        const int mb = mbk_tcg_max_blocks(mixed);
-        m->pcg.blocks = items < mb ? items : mb;
-    } else if (bestc == nv + 1) {
-        m->pcg.form = MB_PCG_RESIDENT;
-        m->pcg.blocks = m->pcg.rc_nbx * m->pcg.rc_nby;
-    } else if (bestc >= f0) {
-        m->pcg.form = MB_PCG_FUSED;
-        m->pcg.variant = bestc - f0;
-        m->pcg.blocks = mbk_ffcg_max_blocks(mixed, kind, m->pcg.variant);
-    } else if (bestc >= c0) {
-        m->pcg.form = MB_PCG_CLUSTER;
-        m->pcg.cc_variant = bestc - c0;
-        m->pcg.blocks = 1 << m->pcg.cc_variant;
-    } else {
-        m->pcg.form = MB_PCG_ZMARCH;
-        m->pcg.zc_variant = bestc - nv - 2;
-        m->pcg.blocks = mbk_zcg_max_blocks(mixed, m->pcg.zc_variant);
-    }
+    m->pcg = win;
     if (m->pcg.form != MB_PCG_FUSED && m->d_apb) {
         cudaFree(m->d_apb);
         m->d_apb = NULL;
@@ -626,14 +655,9 @@ static int cg_autotune(mb_monodomain *m) {
     if (m->pcg.form != MB_PCG_ZMARCH) {
         cudaFree(m->pcg.zc_xpad);
         cudaFree(m->pcg.zc_vpad);
-        m->pcg.zc_xpad = m->pcg.zc_vpad = NULL;
+        cudaFree(m->pcg.zc_w);
+        m->pcg.zc_xpad = m->pcg.zc_vpad = m->pcg.zc_w = NULL;
     }
-    if (m->pcg.form != MB_PCG_RESIDENT && m->d_rtrue) {
-        cudaFree(m->d_rtrue);
-        m->d_rtrue = NULL;
-        m->pcg.rtrue = NULL;
-    }
-    m->cg_tune_ms = best / 2.0f;
     return MB_OK;
 }
 
@@ -890,31 +914,21 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
     m->cg.partials = m->d_partials;
 
     /* persistent cooperative CG: one launch per solve */
+    int cand[CG_MAX_CANDIDATES], ncand = 0;
     {
         const char *mode = getenv("MB_CG");
         m->use_pcg = !(mode && strcmp(mode, "graph") == 0);
         const int mixed = d->precision == MB_PREC_MIXED;
+        m->pcg.mixed = mixed;
+        m->pcg.st = m->st;
         int maxb = -1;
+        ncand = cg_candidates(m, cand);
         if (m->use_pcg) {
-            /* the partials buffer must fit the largest grid of any variant */
-            const int nv = mbk_fcg_variants(m->st.kind);
-            for (int v = 0; v < nv; ++v) {
-                const int b = mbk_fcg_max_blocks(mixed, m->st.kind, v);
-                if (b > maxb) maxb = b;
+            /* the partials buffer must fit the largest grid of any candidate */
+            for (int k = -1; k < ncand; ++k) {
+                mb_pcg_dev q = m->pcg;
+                if (cg_select(m, k < 0 ? 0 : cand[k], &q) && q.blocks > maxb) maxb = q.blocks;
             }
-            for (int v = 0; mbk_ffcg_usable(&m->st) && v < mbk_ffcg_variants(); ++v) {
-                const int b = mbk_ffcg_max_blocks(mixed, m->st.kind, v);
-                if (b > maxb) maxb = b;
-            }
-            const int bt = mbk_tcg_max_blocks(mixed);
-            if (bt > maxb) maxb = bt;
-            if (mbk_zcg_usable(&m->st))
-                for (int v = 0; v < mbk_zcg_variants(); ++v) {
-                    const int b = mbk_zcg_max_blocks(mixed, v);
-                    if (b > maxb) maxb = b;
-                }
-            mbk_tcg_layout(d->nx, d->ny, d->nz, bt > 0 ? bt : 1, &m->pcg.tiles_x, &m->pcg.tiles_y, &m->pcg.zchunk,
-                           &m->pcg.nchunks);
         }
         if (maxb <= 0) m->use_pcg = 0;
         if (m->use_pcg) {
@@ -966,7 +980,6 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
             CKK(cudaMemset(m->d_bar, 0, 2 * sizeof(unsigned)));
             CKK(cudaMemset(m->d_status, 0, sizeof(int)));
             mb_pcg_dev *q = &m->pcg;
-            q->mixed = d->precision == MB_PREC_MIXED;
             q->form = MB_PCG_FLAT;
             q->variant = 0;
             q->rc_shape = -1;
@@ -985,7 +998,6 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
             q->inv_diag32 = m->d_invd32;
             q->bar = m->d_bar;
             q->status = m->d_status;
-            q->st = m->st;
             if (q->zc_inv64) CKK(mbk_zcg_prepare(q));
         }
     }
@@ -1072,7 +1084,7 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
     m->log_len = 1 << 20;
     ALLOC(m->d_log, (size_t)m->log_len * sizeof(mb_step_stats));
 
-    rc = cg_autotune(m);
+    rc = cg_autotune(m, cand, ncand);
     if (rc) goto fail;
     rc = build_graphs(m);
     if (rc) goto fail;
