@@ -139,6 +139,7 @@ int mbk_ode_step_mixed(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vin, do
 int mbk_ode_init(const mb_ode_dev *o, const double *table_dev, int ntypes, cudaStream_t s);
 int mbk_ode_step(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vin, double *vout,
                  cudaStream_t s);
+int mbk_ode_variants(int model, int precision, int num_steps, int adaptive);
 int mbk_ode_default_variant(int model, int precision, uint32_t n, int num_steps);
 int mbk_ode_gather(const mb_ode_dev *o, const double *v, double *out_dev, cudaStream_t s);
 int mbk_ode_scatter(const mb_ode_dev *o, const double *in_dev, double *v, cudaStream_t s);

@@ -1155,7 +1155,8 @@ static int ode_autotune(mb_monodomain *m) {
     t.out_ld = nt;
     float best = 1e30f;
     int bestv = 0;
-    for (int v = 0; v < MB_ODE_VARIANTS && !rc; ++v) {
+    const int nv = mbk_ode_variants(t.model, t.precision, t.num_steps, t.adaptive);
+    for (int v = 0; v < nv && !rc; ++v) {
         t.variant = v;
         const int e = mbk_ode_step(&t, NULL, m->d_vstar, vs, m->stream);
         if (e == (int)cudaErrorInvalidConfiguration && v >= 6) continue;   /* staged form does not fit */

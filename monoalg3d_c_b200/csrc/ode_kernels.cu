@@ -194,6 +194,13 @@ extern "C" int mbk_ode_step(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vi
     return (int)cudaGetLastError();
 }
 
+// Variants 0 .. count - 1 are the ones that launch different kernels.
+extern "C" int mbk_ode_variants(int model, int precision, int num_steps, int adaptive) {
+    if (model == MB_MODEL_TORORD_FKATP_ENDO) return adaptive ? 1 : 4;
+    if (model == MB_MODEL_TT2006 || num_steps == 1) return MB_ODE_VARIANTS;
+    return precision == MB_PREC_FP64 ? 4 : 2;
+}
+
 // The variant of an object that is not tuned (mb_ode_create).  Up to two
 // blocks per SM the register budget does not limit what runs at once, so the
 // kernel with the most registers is taken; beyond that FP64 takes 128 registers
@@ -201,7 +208,7 @@ extern "C" int mbk_ode_step(const mb_ode_dev *o, mb_ctrl *ctrl, const double *vi
 // occupancy that does not spill.
 extern "C" int mbk_ode_default_variant(int model, int precision, uint32_t n, int num_steps) {
     if (model == MB_MODEL_TORORD_FKATP_ENDO) return 0;
-    if ((n + ODE_THREADS - 1) / ODE_THREADS <= 2 * 148) return 0;
+    if ((n + ODE_THREADS - 1) / ODE_THREADS <= (unsigned)mbk_max_grid_blocks() / 4) return 0;   // 8 per SM
     if (precision == MB_PREC_FP64) return model != MB_MODEL_TT2006 && num_steps > 1 ? 0 : 3;
     if (model == MB_MODEL_TT2006) return 5;
     return num_steps > 1 ? 1 : 4;
