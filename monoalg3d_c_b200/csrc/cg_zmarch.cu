@@ -1386,9 +1386,10 @@ constexpr Variant make() {
     return {(const void *)k_zcg<MIXED, W, S, MINB, MODE>, W, Lay<typename Prec<MIXED>::T, W, S, MODE>::BYTES, MODE};
 }
 
-// Mixed: 4-6 run the window Q pass, 7-9 the fused pass.  FP64 has neither
-// (its iterations keep the U pass, whose r.r decides the stop exactly as the
-// reference's loop does); its 4-6 are ring-pass shapes whose shared memory
+// Mixed: 4-6 run the window Q pass, 7-9 the fused pass.  FP64 has neither: the
+// fused pass has no guard against cancellation of its recurred r.r, which in FP64
+// decides the stop itself (in mixed precision the FP64 residual does; the flat fused and
+// the cluster kernel have the guard and stop on the recurred sum); its 4-6 are ring-pass shapes whose shared memory
 // fits (four stages of FP64 planes of W = 16 do not) and 7-9 are empty.
 constexpr int NUM_VARIANTS = 10;
 
@@ -1542,13 +1543,7 @@ extern "C" int mbk_zcg_ptab_floats(void) { return PTAB; }
 extern "C" int mbk_zcg_prepare(mb_pcg_dev *p) {
     const int nx = padded_nx(&p->st), ny = p->st.ny, nz = p->st.nz;
     const int elem = p->mixed ? 4 : 8;
-    if (nx != p->st.nx) {
-        const size_t bytes = (size_t)nx * ny * nz * sizeof(double);
-        cudaError_t e = cudaSuccess;
-        if (!p->zc_xpad) e = cudaMalloc((void **)&p->zc_xpad, bytes);
-        if (e == cudaSuccess && !p->zc_vpad) e = cudaMalloc((void **)&p->zc_vpad, bytes);
-        if (e != cudaSuccess) return (int)e;
-    }
+    if (nx != p->st.nx && (!p->zc_xpad || !p->zc_vpad)) return (int)cudaErrorInvalidValue;
     alignas(64) CUtensorMap tm[NUM_VARIANTS * MAPS];
     memset(tm, 0, sizeof tm);
     const void *bases[MAPS] = {p->mixed ? (const void *)p->r32 : (const void *)p->r64,
@@ -1635,6 +1630,8 @@ extern "C" int mbk_zcg_launch(const mb_pcg_dev *p, cudaStream_t s) {
         a.x = p->zc_xpad;
         a.vstar = p->zc_vpad;
         k_pad<<<1184, 256, 0, s>>>(p->zc_xpad, p->x, p->zc_vpad, p->vstar, p->st.nx, nx, rows);
+        const cudaError_t pe = cudaGetLastError();
+        if (pe != cudaSuccess) return (int)pe;
     }
     a.r64 = p->r64; a.pa64 = p->pa64; a.pb64 = p->pb64; a.z64 = p->z64;
     a.r32 = p->r32; a.pa32 = p->pa32; a.pb32 = p->pb32; a.z32 = p->z32;

@@ -489,7 +489,8 @@ static int cg_select(const mb_monodomain *m, int cand, mb_pcg_dev *q) {
     if (cand >= cg_number(CG_FUSED)) {
         q->form = MB_PCG_FUSED;
         q->variant = cand - cg_number(CG_FUSED);
-        if (!mbk_ffcg_usable(&m->st) || (mbk_ffcg_variant_groups(q->variant) && !whole)) return 0;
+        if (!(mixed ? (void *)m->d_ap32b : (void *)m->d_apb) || !mbk_ffcg_usable(&m->st)) return 0;
+        if (mbk_ffcg_variant_groups(q->variant) && !whole) return 0;
         q->blocks = mbk_ffcg_max_blocks(mixed, kind, q->variant);
     } else if (cand >= cg_number(CG_CLUSTER)) {
         q->form = MB_PCG_CLUSTER;
@@ -499,7 +500,7 @@ static int cg_select(const mb_monodomain *m, int cand, mb_pcg_dev *q) {
     } else if (cand >= cg_number(CG_ZMARCH)) {
         q->form = MB_PCG_ZMARCH;
         q->zc_variant = cand - cg_number(CG_ZMARCH);
-        if (!mbk_zcg_variant_usable(&m->st, mixed, q->zc_variant)) return 0;
+        if (!q->zc_maps || !mbk_zcg_variant_usable(&m->st, mixed, q->zc_variant)) return 0;
         q->blocks = mbk_zcg_max_blocks(mixed, q->zc_variant);
     } else if (cand == cg_number(CG_RESIDENT)) {
         if (!mbk_rcg_plan(q)) return 0;
@@ -539,9 +540,10 @@ static int cg_select(const mb_monodomain *m, int cand, mb_pcg_dev *q) {
  *     2 M 939 / 632, flat 1031 / 669; 25 M 8620 / 4530, flat 11400 / 7400), ragged rows
  *     shape 0 too (500 k 470 / 366, flat 383 / 391); clusters to 8 k cells (4000 cells
  *     162, z-march 172 / 178).
- * The tiled and the resident kernel win nowhere any more; they run by number. */
+ * The tiled and the resident kernel win nowhere any more; they run by number.
+ * zmarch 0: without the z-march variants (no room for their vectors). */
 enum { CG_MAX_CANDIDATES = 12 };
-static int cg_candidates(const mb_monodomain *m, int *list) {
+static int cg_candidates(const mb_monodomain *m, int zmarch, int *list) {
     const int z0 = cg_number(CG_ZMARCH), c0 = cg_number(CG_CLUSTER), f0 = cg_number(CG_FUSED);
     const int mixed = m->desc.precision == MB_PREC_MIXED, wide = m->st.kind == 2, whole = m->desc.nx % 4 == 0;
     int n = 0;
@@ -556,7 +558,7 @@ static int cg_candidates(const mb_monodomain *m, int *list) {
         list[n++] = c0 + v;
         if (v + 1 < mbk_ccg_variants()) list[n++] = c0 + v + 1;
     }
-    if (wide && mbk_zcg_usable(&m->st)) {
+    if (zmarch && mbk_zcg_usable(&m->st)) {
         static const int z64[] = {0, 2, 5}, z32[] = {7, 8, 9, 0, 1};
         for (int k = 0; k < (mixed ? 5 : 3); ++k) list[n++] = z0 + (mixed ? z32[k] : z64[k]);
         list[n++] = 12;
@@ -571,6 +573,48 @@ static int cg_candidates(const mb_monodomain *m, int *list) {
         for (int k = 0; k < (few ? 1 : whole ? 6 : 4); ++k) list[n++] = whole ? vec[k] : one[k];
     }
     return n;
+}
+
+/* The CG's vectors, zeroed: the ones every form uses and, as asked for, those of the z-march
+ * kernel (whose rows may be padded) and the second A p of the fused forms.  All or none. */
+static cudaError_t cg_vectors(mb_monodomain *m, int zmarch, int fused) {
+    const int mixed = m->desc.precision == MB_PREC_MIXED;
+    const size_t n = (size_t)m->n, nc = zmarch ? (size_t)mbk_zcg_cells(&m->st) : n, nz = (size_t)m->desc.nz;
+    const size_t w = nc * (mixed ? sizeof(float) : sizeof(double)), pcg = m->use_pcg ? w : 0;
+    const struct { void **p; size_t bytes; } v[] = {
+        {mixed ? (void **)&m->d_r32 : (void **)&m->d_r, w},
+        {mixed ? (void **)&m->d_p32 : (void **)&m->d_p, w},
+        {mixed ? (void **)&m->d_pb32 : (void **)&m->d_pb, pcg},
+        {mixed ? (void **)&m->d_z32 : (void **)&m->d_z, pcg},
+        {mixed ? (void **)&m->d_ap32 : (void **)&m->d_ap, pcg},
+        {mixed ? (void **)&m->d_invd32 : (void **)&m->d_invd, m->use_pcg ? n * (mixed ? sizeof(float) : sizeof(double)) : 0},
+        {mixed ? (void **)&m->d_ap32b : (void **)&m->d_apb, fused || (zmarch && mixed) ? w : 0},
+        {(void **)&m->pcg.zc_inv64, zmarch ? nz * 9 * sizeof(double) : 0},
+        {(void **)&m->pcg.zc_inv32, zmarch ? nz * 9 * sizeof(float) : 0},
+        {(void **)&m->pcg.zc_ptab32, zmarch ? nz * mbk_zcg_ptab_floats() * sizeof(float) : 0},
+        /* A x of the fused mixed solve's last residual (its next solve's starting product) */
+        {(void **)&m->pcg.zc_w, zmarch && mixed ? nc * sizeof(double) : 0},
+        {(void **)&m->pcg.zc_xpad, nc != n ? nc * sizeof(double) : 0},
+        {(void **)&m->pcg.zc_vpad, nc != n ? nc * sizeof(double) : 0},
+    };
+    cudaError_t e = cudaSuccess;
+    for (size_t k = 0; k < sizeof v / sizeof v[0]; ++k) {
+        cudaFree(*v[k].p);
+        *v[k].p = NULL;
+    }
+    for (size_t k = 0; k < sizeof v / sizeof v[0] && e == cudaSuccess; ++k) {
+        if (!v[k].bytes) continue;
+        e = cudaMalloc(v[k].p, v[k].bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(*v[k].p, 0, v[k].bytes, m->stream);
+    }
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();
+    cudaStreamSynchronize(m->stream);
+    for (size_t k = 0; k < sizeof v / sizeof v[0]; ++k) {
+        cudaFree(*v[k].p);
+        *v[k].p = NULL;
+    }
+    return e;
 }
 
 /* Picks the CG kernel: the candidates solve one system; V is restored after every trial
@@ -886,8 +930,6 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
     m->st.rowid = m->d_rowid;
     CKK(mbk_stencil_codes(&m->st, m->d_code, m->d_rowid, m->stream));
 
-    /* CG work vectors (the z-march kernel's rows may be padded) */
-    const int64_t nc = mbk_zcg_cells(&m->st);
     m->cg.precision = d->precision;
     {
         int gb = (int)((n + 255) / 256);
@@ -896,22 +938,6 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
         m->cg.grid_blocks = gb;
         ALLOC(m->d_partials, (size_t)3 * gb * sizeof(double));
     }
-    if (d->precision == MB_PREC_FP64) {
-        ALLOC(m->d_r, (size_t)nc * sizeof(double));
-        ALLOC(m->d_p, (size_t)nc * sizeof(double));
-        CKK(cudaMemset(m->d_r, 0, (size_t)nc * sizeof(double)));
-        CKK(cudaMemset(m->d_p, 0, (size_t)nc * sizeof(double)));
-    } else {
-        ALLOC(m->d_r32, (size_t)nc * sizeof(float));
-        ALLOC(m->d_p32, (size_t)nc * sizeof(float));
-        CKK(cudaMemset(m->d_r32, 0, (size_t)nc * sizeof(float)));
-        CKK(cudaMemset(m->d_p32, 0, (size_t)nc * sizeof(float)));
-    }
-    m->cg.x = m->d_v;
-    m->cg.vstar = m->d_vstar;
-    m->cg.r = m->d_r; m->cg.p = m->d_p;
-    m->cg.r32 = m->d_r32; m->cg.p32 = m->d_p32;
-    m->cg.partials = m->d_partials;
 
     /* persistent cooperative CG: one launch per solve */
     int cand[CG_MAX_CANDIDATES], ncand = 0;
@@ -921,60 +947,39 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
         const int mixed = d->precision == MB_PREC_MIXED;
         m->pcg.mixed = mixed;
         m->pcg.st = m->st;
-        int maxb = -1;
-        ncand = cg_candidates(m, cand);
+        if (m->use_pcg && mbk_fcg_max_blocks(mixed, m->st.kind, 0) <= 0) m->use_pcg = 0;
+        /* the candidates and their vectors; without the vectors that only the z-march and
+         * the fused kernels use where there is no room for them */
+        int zmarch = 0, fused = 0;
         if (m->use_pcg) {
-            /* the partials buffer must fit the largest grid of any candidate */
-            for (int k = -1; k < ncand; ++k) {
-                mb_pcg_dev q = m->pcg;
-                if (cg_select(m, k < 0 ? 0 : cand[k], &q) && q.blocks > maxb) maxb = q.blocks;
+            ncand = cg_candidates(m, 1, cand);
+            for (int k = 0; k < ncand; ++k) {
+                if (cand[k] >= cg_number(CG_FUSED)) fused |= mbk_ffcg_usable(&m->st);
+                else if (cand[k] >= cg_number(CG_ZMARCH) && cand[k] < cg_number(CG_CLUSTER))
+                    zmarch |= mbk_zcg_variant_usable(&m->st, mixed, cand[k] - cg_number(CG_ZMARCH));
             }
         }
-        if (maxb <= 0) m->use_pcg = 0;
+        cudaError_t e = cg_vectors(m, zmarch, fused);
+        if (e == cudaSuccess && zmarch && mbk_zcg_cells(&m->st) != n) {
+            /* padded rows: leave what the rest of the creation and the pipelined host calls need */
+            size_t fr = 0, tot = 0;
+            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr < (size_t)n * 48 + ((size_t)64 << 20)) e = cudaErrorMemoryAllocation;
+        }
+        if (e != cudaSuccess && (zmarch || fused)) {
+            zmarch = fused = 0;
+            ncand = cg_candidates(m, 0, cand);
+            e = cg_vectors(m, 0, 0);
+        }
+        if (e != cudaSuccess) {
+            rc = set_err(MB_ERR_NOMEM, "CG vectors: %s", cudaGetErrorString(e));
+            goto fail;
+        }
+        m->cg.x = m->d_v;
+        m->cg.vstar = m->d_vstar;
+        m->cg.r = m->d_r; m->cg.p = m->d_p;
+        m->cg.r32 = m->d_r32; m->cg.p32 = m->d_p32;
+        m->cg.partials = m->d_partials;
         if (m->use_pcg) {
-            const int blocks = maxb;
-            if (d->precision == MB_PREC_FP64) {
-                ALLOC(m->d_pb, (size_t)nc * sizeof(double));
-                CKK(cudaMemset(m->d_pb, 0, (size_t)nc * sizeof(double)));
-                ALLOC(m->d_z, (size_t)nc * sizeof(double));
-                CKK(cudaMemset(m->d_z, 0, (size_t)nc * sizeof(double)));
-                ALLOC(m->d_ap, (size_t)nc * sizeof(double));
-                CKK(cudaMemset(m->d_ap, 0, (size_t)nc * sizeof(double)));
-                if (mbk_ffcg_usable(&m->st)) {
-                    ALLOC(m->d_apb, (size_t)n * sizeof(double));
-                    CKK(cudaMemset(m->d_apb, 0, (size_t)n * sizeof(double)));
-                }
-            } else {
-                ALLOC(m->d_pb32, (size_t)nc * sizeof(float));
-                CKK(cudaMemset(m->d_pb32, 0, (size_t)nc * sizeof(float)));
-                ALLOC(m->d_z32, (size_t)nc * sizeof(float));
-                CKK(cudaMemset(m->d_z32, 0, (size_t)nc * sizeof(float)));
-                ALLOC(m->d_ap32, (size_t)nc * sizeof(float));
-                CKK(cudaMemset(m->d_ap32, 0, (size_t)nc * sizeof(float)));
-                if (mbk_zcg_usable(&m->st) || mbk_ffcg_usable(&m->st)) {
-                    /* the fused passes alternate A p between two buffers */
-                    ALLOC(m->d_ap32b, (size_t)nc * sizeof(float));
-                    CKK(cudaMemset(m->d_ap32b, 0, (size_t)nc * sizeof(float)));
-                }
-            }
-            ALLOC(m->d_ppart, ((size_t)16 * blocks + 16) * sizeof(double));
-            if (d->precision == MB_PREC_FP64) {
-                ALLOC(m->d_invd, (size_t)n * sizeof(double));
-                CKK(cudaMemset(m->d_invd, 0, (size_t)n * sizeof(double)));
-            } else {
-                ALLOC(m->d_invd32, (size_t)n * sizeof(float));
-                CKK(cudaMemset(m->d_invd32, 0, (size_t)n * sizeof(float)));
-            }
-            CKK(mbk_inv_diag(&m->st, m->d_invd, m->d_invd32, m->stream));
-            if (mbk_zcg_usable(&m->st)) {
-                ALLOC(m->pcg.zc_inv64, (size_t)d->nz * 9 * sizeof(double));
-                ALLOC(m->pcg.zc_inv32, (size_t)d->nz * 9 * sizeof(float));
-                ALLOC(m->pcg.zc_ptab32, (size_t)d->nz * mbk_zcg_ptab_floats() * sizeof(float));
-                /* the fused mixed solve's stored A x (its next solve's starting product) */
-                if (d->precision == MB_PREC_MIXED) ALLOC(m->pcg.zc_w, (size_t)nc * sizeof(double));
-                CKK(mbk_zcg_inv_tables(&m->st, m->pcg.zc_inv64, m->pcg.zc_inv32, m->pcg.zc_ptab32, m->stream));
-            }
-            CKK(cudaStreamSynchronize(m->stream));
             ALLOC(m->d_bar, 2 * sizeof(unsigned));
             ALLOC(m->d_status, sizeof(int));
             CKK(cudaMemset(m->d_bar, 0, 2 * sizeof(unsigned)));
@@ -993,12 +998,29 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
             q->z64 = m->d_z; q->z32 = m->d_z32;
             q->ap64 = m->d_ap; q->ap32 = m->d_ap32; q->ap32b = m->d_ap32b;
             q->ap64b = m->d_apb;
-            q->partials = m->d_ppart;
             q->inv_diag64 = m->d_invd;
             q->inv_diag32 = m->d_invd32;
             q->bar = m->d_bar;
             q->status = m->d_status;
-            if (q->zc_inv64) CKK(mbk_zcg_prepare(q));
+            CKK(mbk_inv_diag(&m->st, m->d_invd, m->d_invd32, m->stream));
+            if (zmarch) {
+                int z = mbk_zcg_inv_tables(&m->st, q->zc_inv64, q->zc_inv32, q->zc_ptab32, m->stream);
+                if (!z) z = mbk_zcg_prepare(q);
+                if (z) {
+                    cudaGetLastError();
+                    cudaFree(q->zc_maps);
+                    q->zc_maps = NULL;
+                }
+            }
+            CKK(cudaStreamSynchronize(m->stream));
+            /* the partials buffer must fit the largest grid of any candidate */
+            int blocks = q->blocks;
+            for (int k = 0; k < ncand; ++k) {
+                mb_pcg_dev t = m->pcg;
+                if (cg_select(m, cand[k], &t) && t.blocks > blocks) blocks = t.blocks;
+            }
+            ALLOC(m->d_ppart, ((size_t)16 * blocks + 16) * sizeof(double));
+            q->partials = m->d_ppart;
         }
     }
 
@@ -1107,6 +1129,7 @@ int mb_monodomain_create(mb_monodomain **out, const mb_monodomain_desc *d) {
     *out = m;
     return MB_OK;
 fail:
+    cudaGetLastError();         /* an allocation's failure is not the next call's */
     free(cells); free(bits); free(ct); free(scale); free(vinit);
     mb_assembly_free(&asmb);
     mb_monodomain_destroy(m);
