@@ -1,7 +1,8 @@
-"""The staged persistent ODE kernels (ODE variants 6..9: each thread copies
-its next cell's state rows into shared memory with cp.async while it
-integrates the current one) against the one-cell-per-thread kernels
-(variant 0), for both models and both precisions, on a grid with removed
+"""Every ODE variant against variant 0: the other register budgets of the
+one-cell-per-thread kernels (1..5), the mixed ToRORd kernel over shared-memory slots
+(its 2..5) and the staged persistent kernels (6..9: each thread copies its next
+cell's state rows into shared memory with cp.async while it integrates the current
+one), for both models and both precisions, on a grid with removed
 cells (compact cell indexing) and a stimulus, large enough that every block
 loops over several tiles.  They run the same per-cell arithmetic, so the bar
 is bit-identical V and state."""
@@ -43,11 +44,11 @@ def _run(model, precision, variant):
 
 @pytest.mark.parametrize("model,precision", [("tt2006", "fp64"), ("tt2006", "mixed"),
                                              ("torord", "fp64"), ("torord", "mixed")])
-def test_staged_variants_match_plain(model, precision):
+def test_variants_match_plain(model, precision):
     v0, s0 = _run(model, precision, 0)
     assert np.isfinite(s0).all()
     ok = np.isfinite(v0)
-    for variant in (6, 7, 8, 9):
+    for variant in range(1, 10):
         v, s = _run(model, precision, variant)
         dv = np.abs(v[ok] - v0[ok])
         ds = np.abs(s - s0) / (np.abs(s0) + 1e-30)
