@@ -524,23 +524,25 @@ static int cg_select(const mb_monodomain *m, int cand, mb_pcg_dev *q) {
 
 /* The kernels that are timed for a tissue (at most CG_MAX_CANDIDATES numbers), those
  * first that mostly win.  Creating a small tissue costs as much as hundreds of its
- * steps, so the rule leaves out what is never the fastest, or by 2 % at most; measured on
- * 56 tissues from 30 to 25 M cells in both precisions (us per solve, FP64 / mixed):
+ * steps, so the rule leaves out what is never the fastest, or by 3 % at most; measured on
+ * 56 tissues from 30 to 25 M cells in both precisions and compared with timing every
+ * kernel on 280 more (us per solve, FP64 / mixed):
  *   7-point, to 32 k cells: the cluster of 340 to 680 cells a block and the next larger
  *     (400 cells 34 / 37, fused 51 / 69; 4096 cells 47 / 48, fused 72 / 87; 16 k cells
  *     72, fused 76); at 65 k cells a cluster takes 111 / 114, the fused form 82 / 95;
  *   7-point, to 2^20 cells: fused shape 0 and, with whole groups of 4 cells in a row,
  *     shape 2, where a flat shape comes last to 2^18 cells (200 k 132 / 132, flat
  *     144 / 137; 262 k 142 / 138, flat 158 / 147) and first from then on (400 k 199 / 217,
- *     flat 225 / 201; 983 k 339 / 262, flat 342 / 246);
+ *     flat 225 / 201; 983 k 339 / 262, flat 342 / 246); mixed with ragged rows from 2^17
+ *     cells on the resident kernel too (223 k 127, fused 133);
  *   beyond: the flat shapes, with whole groups those of 4 cells a thread (2 M 602 / 366,
  *     25 M 7500 / 4480), for a plane in FP64 one cell a thread (1 M 250, groups 291),
  *     else one cell a thread (2 M 613 / 419);
- *   27-point: the z-march variants and flat shape 12 (19 k cells 176 / 179, flat 176 / 186;
- *     2 M 939 / 632, flat 1031 / 669; 25 M 8620 / 4530, flat 11400 / 7400), ragged rows
- *     shape 0 too (500 k 470 / 366, flat 383 / 391); clusters to 8 k cells (4000 cells
- *     162, z-march 172 / 178).
- * The tiled and the resident kernel win nowhere any more; they run by number.
+ *   27-point: the z-march variants and a few flat shapes (19 k cells 176 / 179, flat
+ *     176 / 186; 469 k with 19 planes 139 mixed on a flat shape, z-march 166; 500 k ragged
+ *     470 / 366, flat 383 / 391; 2 M 939 / 632, flat 1031 / 669; 25 M 8620 / 4530, flat
+ *     11400 / 7400); clusters to 8 k cells (4000 cells 162, z-march 172 / 178).
+ * The tiled kernel wins nowhere any more and runs by number.
  * zmarch 0: without the z-march variants (no room for their vectors). */
 enum { CG_MAX_CANDIDATES = 12 };
 static int cg_candidates(const mb_monodomain *m, int zmarch, int *list) {
@@ -559,16 +561,17 @@ static int cg_candidates(const mb_monodomain *m, int zmarch, int *list) {
         if (v + 1 < mbk_ccg_variants()) list[n++] = c0 + v + 1;
     }
     if (zmarch && mbk_zcg_usable(&m->st)) {
-        static const int z64[] = {0, 2, 5}, z32[] = {7, 8, 9, 0, 1};
+        static const int z64[] = {0, 2, 5}, z32[] = {9, 8, 7, 1, 0};
         for (int k = 0; k < (mixed ? 5 : 3); ++k) list[n++] = z0 + (mixed ? z32[k] : z64[k]);
-        list[n++] = 12;
-        if (!whole) list[n++] = 0;
+        static const int flat[] = {12, 0, 17, 22};
+        for (int k = 0; k < (whole ? 4 : 2); ++k) list[n++] = flat[k];
     } else {
         static const int vec[] = {22, 10, 17, 8, 20, 0}, one[] = {12, 14, 0, 2};
         const int few = mbk_ffcg_usable(&m->st) && m->n <= (1 << 18);
         if (mbk_ffcg_usable(&m->st)) {
             list[n++] = f0;
             if (whole) list[n++] = f0 + 2;
+            else if (mixed && m->n > (1 << 17)) list[n++] = cg_number(CG_RESIDENT);
         }
         for (int k = 0; k < (few ? 1 : whole ? 6 : 4); ++k) list[n++] = whole ? vec[k] : one[k];
     }
