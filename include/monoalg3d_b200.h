@@ -431,7 +431,8 @@ int mb_monodomain_time_steps_host_async(mb_monodomain *m, int n, const double *s
  * environment variable MB_CG_VARIANT, read at creation, forces a choice:
  * 0..n-1 a flat shape, n the tiled kernel, n + 1 the resident kernel, n + 2 + v
  * z-march variant v (300 + v), then the cluster kernel with 2^v blocks
- * (400 + v), then the fused flat form's shapes (500 + v). */
+ * (400 + v), then the fused flat form's shapes (500 + v); a number that does
+ * not run on the tissue leaves flat shape 0. */
 int mb_monodomain_tuning(mb_monodomain *m, int *ode_variant, int *cg_blocks, int *cg_kernel);
 int mb_cg_launch_shapes(int *flat_shapes);
 

@@ -3,13 +3,13 @@
 // blocks are read through distributed shared memory, and the iteration
 // synchronises with cluster barriers instead of grid reductions through L2.
 //
-// Why: below about 100 k cells an iteration of the grid-wide kernel (cg_flat.cu)
+// Why: below about 100 k cells an iteration of the grid-wide two-pass kernel (cg_flat.cu)
 // is its two grid reductions, 6.5 - 7 us with 148 blocks whether the tissue has 400
-// cells or 65 k.  Here it takes 2.5 us for a 400-cell cable (a solve of 10 iterations
+// cells or 65 k, and of the fused one 5 us.  Here it takes 2.5 us for a 400-cell cable (a solve of 10 iterations
 // 34 us, 66 us grid-wide) and 3.8 us for 12.7 k cells in 16 blocks (61 against 98
 // us for 13), bound by the latency of the reduction's and the rows' FP64
-// chains; with 4 k cells per block (65 k, FP64) a block's work is 5 us and the grid-wide
-// kernel is faster (94 against 104 us), so the host times both.
+// chains; with 4 k cells per block (65 k, FP64) a block's work is 5 us and the fused
+// grid-wide kernel is faster (80 against 111 us): the host times clusters to 32 k cells.
 //
 // One reduction per iteration: with q = A p and z = M r (M the Jacobi
 // preconditioner) the pass sums p.q, q.z, q.Mq, q.r, q.q, r.z and r.r; then

@@ -2,8 +2,8 @@
 configuration at a scale, steps it a few times and prints its tuning and a
 per-phase timing.  Launch choices can be forced through the environment the
 tissue reads at creation: MB_ODE_VARIANT (cell-model kernel) and
-MB_CG_VARIANT (CG form and launch shape: the flat shapes, then the tiled,
-resident and z-march kernels, as `Tissue.tuning()` reports them).
+MB_CG_VARIANT (CG form and launch shape: 0-23 flat, 24 tiled, 25 resident, 26-35
+z-march, 36-40 clusters, 41-43 the fused flat form; `Tissue.tuning()` reports what ran).
 
     python -m monoalg3d_c_b200.profile_run [--config 4] [--scale 0.72] [--precision mixed] [--steps 5]
 
