@@ -8,10 +8,12 @@
 //
 // A part of a warp (LANES lanes) takes a row, so that its entries are read
 // as whole sectors, R rows at a time: bound by the latency of row pointer, entry and
-// vector value, one after the other.  R = 4 fits 64 registers, two blocks per SM; with one
-// row at a time the kernel took 126, one block (22 us), R = 2 took 18 us and R = 8, 106
-// registers, 17 us.  Once matrix and vectors leave L2 this is not enough: the phases'
-// thread per row keeps four times the rows in flight (mbk_csr_in_l2).
+// vector value, one after the other (profiles/k_csr_pcg_200k.md).  R = 4 takes 108
+// registers, one block per SM: 16 us an iteration at 200 k rows, 22 us with one row at a
+// time, 18 and 17 us with R = 2 and 8.  Bound to 64 registers, two blocks per SM, it is
+// faster on large matrices (600 k rows 26 us, 33 here) and slower on small ones (50 k rows 12
+// us, 9 here).  Once matrix and vectors leave L2 a thread per row in the phases' kernels
+// keeps more rows in flight (mbk_csr_in_l2).
 // Per iteration: x, r and p of the rows, a grid barrier (p of
 // other rows is read next), then q = A p and the sums p.q, q.z, q.Mq, q.r, q.q,
 // r.z, r.r for the next r.z and r.r (cg_cluster.cu, with its guard).
