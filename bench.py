@@ -187,9 +187,9 @@ PROFILED_CG_TRAFFIC = {
 PROFILED_ODE = {
     # k_torord_mixed_slots<0, 6> / k_torord_fp64<0, 6> on the 0.72-scale slab
     ("slab_500x500x100_torord_rotating_fibres", "mixed", 4): {
-        "fma_pct": 38.2, "issue_active_pct": 64.0, "dram_bytes_per_cell_step": 411.5, "mufu_per_cell_step": 196.0},
+        "xu_pct": 54.5, "fma_pct": 36.3, "issue_active_pct": 61.9, "dram_bytes_per_cell_step": 411.5, "mufu_per_cell_step": 196.0},
     ("slab_500x500x100_torord_rotating_fibres", "fp64", 5): {
-        "fp64_pipe_pct": 52.2, "issue_active_pct": 56.3, "fp64_ops_per_cell_step": 2132.0, "mufu_per_cell_step": 95.3},
+        "fp64_pipe_pct": 50.9, "issue_active_pct": 56.3, "fp64_ops_per_cell_step": 2127.0, "mufu_per_cell_step": 95.3},
 }
 
 

@@ -8,7 +8,7 @@
 //
 // A part of a warp (LANES lanes) takes a row, so that its entries are read
 // as whole sectors, R rows at a time: bound by the latency of row pointer, entry and
-// vector value, one after the other (profiles/k_csr_pcg_200k.md).  R = 4 takes 108
+// vector value, one after the other.  R = 4 takes 108
 // registers, one block per SM: 16 us an iteration at 200 k rows, 22 us with one row at a
 // time, 18 and 17 us with R = 2 and 8.  Bound to 64 registers, two blocks per SM, it is
 // faster on large matrices (600 k rows 26 us, 33 here) and slower on small ones (50 k rows 12

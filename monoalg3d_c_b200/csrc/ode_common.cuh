@@ -295,8 +295,8 @@ struct TorRegsMixed {
 };
 
 // FP64, one sub-step per call: the rows stream through the step.  Bound by the
-// FP64 pipe and the latency of its chains: 461 us for 2 M cells, the pipe 49 % busy
-// with 2106 FP64 instructions per cell (2237 us and 18 % with 3910 when the 43
+// FP64 pipe and the latency of its chains: 462 us for 2 M cells, the pipe 51 % busy
+// with 2127 FP64 instructions per cell (2237 us and 18 % with 3910 when the 43
 // states and 26 coefficient pairs were held in registers and exp and the
 // divisions were the CUDA library's).
 template <int RULE, int MINB>
@@ -612,7 +612,7 @@ k_torord_mixed_s(mb_ode_dev o, const mb_ctrl *__restrict__ ctrl, const double *v
 // Mixed, one sub-step per call, one tile per block with the rows copied into
 // shared memory first: every load of a cell is in flight at once, as in the
 // register form, at the register budget of the streaming one (80 registers, no
-// spills, 24 warps per SM).  Bound by HBM: 619 us for 8 M cells (416 B each, 83 % of
+// spills, 24 warps per SM).  Bound by HBM: 617 us for 8 M cells (416 B each, 83 % of
 // the measured copy rate) against 658 us for the best register form, 717 us for
 // the best persistent staged one, and 800 us for the register form that held
 // the gates' coefficients as well.
