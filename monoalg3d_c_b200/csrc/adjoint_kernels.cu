@@ -68,8 +68,8 @@ constexpr int ADJ_IN = TT_NEQ + 1;      // the 19 states and the gKr scaling
 // FP32): model values and local derivatives are in T, the adjoint values they
 // are contracted with are FP64.
 //
-// What bounds it is the FP64 pipe and the latency of its chains (a 256 x 256
-// sheet is four warps per scheduler).  The sweep costs about three evaluations
+// What bounds it is the FP64 pipe and the latency of its chains (254 registers, two
+// warps per scheduler).  The sweep costs about three evaluations
 // of the model: 21 us per step on a 256 x 256 sheet in FP64 and 18 us on a
 // 97 x 131 sheet in FP32, against 1876 and 239 us for J column block by column
 // block with forward-mode duals (the model and two tangents, ten times).

@@ -705,6 +705,10 @@ static int cg_autotune(mb_monodomain *m, const int *list, int count) {
         cudaFree(m->pcg.zc_w);
         m->pcg.zc_xpad = m->pcg.zc_vpad = m->pcg.zc_w = NULL;
     }
+    if (m->pcg.form != MB_PCG_RESIDENT) {
+        cudaFree(m->d_rtrue);
+        m->d_rtrue = NULL;
+    }
     return MB_OK;
 }
 
