@@ -71,10 +71,13 @@ __device__ __forceinline__ void tt2006_gate_rates(const T V, const T Ca_ss, T (&
     }
     const T em = sigm(MB_OVER(T(-56.86f) - V, 9.03f));
     inf[3] = em * em;
-    // 1 / (a (0.1 / b + 0.1 / c)), b = 1 + exp((V + 35) / 5), c = 1 + exp((V - 50) / 200): b and c as
-    // reciprocals, because b c overflows from 400 mV on in FP32 and 3.4 V in FP64
-    rate[3] = (T(1.0f) + mexp(MB_OVER(T(-60.0f) - V, 5.0f))) *
-              mrcp(T(0.1f) * (sigm(MB_OVER(V + T(35.0f), 5.0f)) + sigm(MB_OVER(V - T(50.0f), 200.0f))));
+    {
+        // 1 / (a (0.1 / b + 0.1 / c)) with b = 1 + exp((V + 35) / 5) as its reciprocal, because b c
+        // overflows from 400 mV on in FP32 and 3.4 V in FP64
+        const T c = T(1.0f) + mexp(MB_OVER(V - T(50.0f), 200.0f));
+        rate[3] = (T(1.0f) + mexp(MB_OVER(T(-60.0f) - V, 5.0f))) * MB_OVER(c, (double)0.1f) *
+                  mrcp(T(1.0f) + c * sigm(MB_OVER(V + T(35.0f), 5.0f)));
+    }
     const T eh = sigm(MB_OVER(V + T(71.55f), 7.43f));
     inf[4] = eh * eh;
     inf[5] = inf[4];

@@ -60,7 +60,7 @@ def test_kernels_not_chosen_keep_no_memory(monkeypatch, rotating):
     other candidates: as much as when that kernel is the only one."""
     torch = pytest.importorskip("torch")
     from monoalg3d_c_b200 import Stim, Tissue
-    nx, ny, nz = 401, 63, 24
+    nx, ny, nz = 401, 101, 24
     kw = dict(assembly="anisotropic", sigma_l=0.0002, sigma_t=0.00004,
               fibre_angle_z=np.deg2rad(np.linspace(60.0, -60.0, nz))) if rotating else {}
 
